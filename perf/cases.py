@@ -4,7 +4,7 @@ A case is a plain dict.  `listed()` names the representative ones, `draw(rng)` g
 same ranges, `prepare(case, seed)` makes what a serving process holds before a call (weights, adapters,
 routed tokens), `run(state)` is one pass through the public entry points, `work(case)` the bytes and
 operations that pass cannot do without, `tolerance(case)` how far another correct implementation of
-the same precision may be from it.
+the same precision may be from it, `exact(case, seed)` the results of a pass in 64 bits.
 
 Ops (the field "op"):
   matmul  matmul_4bit_2_4         one packed int4 2:4 weight, T tokens
@@ -253,3 +253,51 @@ def tolerance(case):
     if case.get("dtype") == "bf16":
         return {"rel": 1e-2, "max": 6e-2}
     return {"rel": 1.2e-3, "max": 8e-3}
+
+
+# -------------------------------------------------------------------------------------------- exact
+def _dense(q, meta, s):
+    """Packed weight -> float64 [K, N], from the storage format alone.  A word of 8 codes serves 8 output columns and 16
+    stored rows per slab; a metadata nibble holds the two kept positions of a group of four along K."""
+    kt, n = q.shape[0], q.shape[1] // 2
+    codes = (q.view(kt, n // 64, 8, 4, 4, 1) >> torch.arange(0, 32, 4, device=q.device, dtype=torch.int32)) & 15
+    codes = codes.view(kt, n // 64, 8, 4, 4, 2, 2, 2)               # slab, block, lane / 4, lane % 4, word, and 3 bits of the nibble
+    levels = codes.permute(0, 7, 3, 5, 1, 2, 6, 4).reshape(kt * 8, 2, n) - 8
+    r = torch.arange(n, device=q.device)[:, None]
+    c = torch.arange(kt * 2, device=q.device)[None, :]
+    at = r // 64 * 64 + r % 2 * 2 + r % 8 // 4 + r % 4 // 2 * 32 + r % 64 // 8 * 4
+    swap = ((at % 2 == 0) & (c % 2 == 1)).long() - ((at % 2 == 1) & (c % 2 == 0)).long()
+    at, c = at + swap, c - swap
+    words = meta.reshape(-1)[c // 2 * n * 2 + at * 2 + c % 2].int()[:, :, None]
+    nibbles = ((words >> torch.arange(0, 16, 4, device=q.device, dtype=torch.int32)) & 15).reshape(n, kt * 8)
+    place = torch.stack([nibbles & 3, nibbles >> 2], 1).permute(2, 1, 0).long()
+    w = torch.zeros(kt * 8, 4, n, dtype=torch.float64, device=q.device).scatter_(1, place, levels.double()).view(kt * 32, n)
+    scale = s.double()
+    if s.shape[0] > 1:                          # group scales: every 8 columns are stored in the order 0 4 1 5 2 6 3 7
+        scale = scale.view(-1, n // 8, 4, 2).transpose(2, 3).reshape(-1, n)
+    return (w.view(s.shape[0], -1, n) * scale[:, None, :]).view(-1, n)
+
+
+def exact(case, seed):
+    """What `run` returns for these inputs, in 64 bits."""
+    st = prepare(case, seed)
+    if case["op"] == "matmul":
+        return st["x"].double() @ _dense(st["q"], st["meta"], st["s"])
+    ids = st["ids"].cpu().numpy()
+    rows = {int(d): torch.from_numpy(np.flatnonzero(ids == d)).cuda() for d in np.unique(ids) if d >= 0}
+    if case["op"] == "stack":
+        sums = torch.zeros(case["T"], dtype=torch.float64, device="cuda")
+        for lin in [lin for layer in st["stack"].layers for lin in layer]:
+            y = torch.empty(case["T"], lin.n, dtype=torch.float64, device="cuda")
+            for d, at in rows.items():
+                y[at] = st["x"][lin.k][at].double() @ _dense(lin.qweights[d], lin.metas[d], lin.scales[d])
+            sums += y.sum(1)
+        return y, sums
+    x, m = st["x"].double(), case.get("M", 0)
+    y = torch.zeros(case["T"], case["N"], dtype=torch.float64, device="cuda") if st["base"] is None else x @ st["base"].double().t()
+    for d, at in rows.items():
+        if d < m:
+            y[at] += x[at] @ st["A"][d].double() @ st["B"][d].double()
+        else:
+            y[at] += x[at] @ _dense(st["q"][d - m], st["meta"][d - m], st["s"][d - m])
+    return y
