@@ -833,6 +833,26 @@ def test_base_gemm_with_lora_expand(cuda, M, rank):
     assert _lib().device_status(0) == 0
 
 
+@pytest.mark.parametrize("groupsize", [-1, 128])
+@pytest.mark.parametrize("K,N", [(128, 384), (896, 512)])
+@pytest.mark.parametrize("counts", [(33, 64, 65), (128, 129, 40), (256, 257, 1), (385, 63, 192)])
+def test_sbmm_token_tile_classes(cuda, counts, K, N, groupsize):
+    """The tcgen05 kernel's 64-, 128- and 256-token tiles at their borders, in lists that mix them (two small
+    accumulators in turn, one large), with one chunk of K and with more than its stages, and with an output
+    whose last stripe is half empty.  Against the oracle; fp16 rounding of the output, of scaled weights
+    and of K <= 896 products bounds the error (ROW_TOL)."""
+    ops = _ops()
+    qs, metas, ss = packed(N, K, groupsize, seed=len(counts) + counts[0], num=4)
+    idx_np = np.repeat(np.array([0, 2, 3]), counts).astype(np.int32)
+    idx_np = np.concatenate([idx_np, np.full(9, -1, np.int32)])
+    idx_np = np.random.default_rng(counts[0]).permutation(idx_np)
+    x = torch.randn(len(idx_np), K, dtype=torch.float16, device=cuda, generator=torch.Generator(cuda).manual_seed(3))
+    idx = torch.from_numpy(idx_np).to(cuda)
+    y = ops.sbmm_4bit_2_4_native(qs, x, metas, ss, idx)
+    check(y, sbmm_ref(qs, metas, ss, x, idx, None))
+    assert _lib().device_status(0) == 0
+
+
 # ------------------------------------------------------------------ tiles chosen per segment, long lists
 def test_sbmm_zipf_batch_mixed_tiles(cuda):
     """A Zipf(1.5) batch of 512 tokens over 64 deltas through the one-call path: the hot deltas

@@ -115,20 +115,35 @@ static int launch_cfg(const GemmCall& c, const GemmArgs& a) {
                                                                                                              : TRB_ERR_CUDA;
 }
 
+// Activations [rows, K] for the sparse tcgen05 kernel: dimensions (64 K, row, 64-K half), a box = `box_rows`
+// rows of two neighbouring halves, each half a 128-byte-swizzled block.
+static bool make_map_x3(CUtensorMap* map, const void* base, uint64_t rows, uint64_t K, uint32_t box_rows) {
+  auto fn = get_encode_fn();
+  if (!fn) return false;
+  cuuint64_t dims[3] = {64, rows, K / 64};
+  cuuint64_t strides[2] = {K * 2, 128};
+  cuuint32_t box[3] = {64, box_rows, 2};
+  cuuint32_t estr[3] = {1, 1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // Prefill-sized tiles: the sparse tcgen05 / TMEM kernel.
-template <class Cfg, class Kernel>
-static int launch_tc_impl(Kernel kernel, const GemmCall& c, const GemmArgs& a) {
+static int launch_tc(const GemmCall& c, const GemmArgs& a) {
+  using Cfg = TcSpCfg;
+  // The sparse kernel writes y in 16-byte pieces of 8 output features.
+  if ((reinterpret_cast<uintptr_t>(a.y) & 15) != 0 || (a.N & 7) != 0) return TRB_ERR_KERN_SHAPE;
   const int slabs = a.K / 32;
   const int groups = a.grouped ? a.K / 128 : 1;
-  CUtensorMap tx, tq, tm, ts;
-  if (!make_map_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, c.x, (uint64_t)a.rows, (uint64_t)a.K, Cfg::B_ROWS, 64,
-                   CU_TENSOR_MAP_SWIZZLE_128B))
-    return TRB_ERR_CUDA;
-  if (!make_map_2d(&tq, CU_TENSOR_MAP_DATA_TYPE_INT32, 4, c.q, (uint64_t)c.num_deltas * slabs, 2ull * a.N, 2, 256,
+  CUtensorMap tx[3], tq, tm, ts;
+  for (int i = 0; i < 3; ++i)
+    if (!make_map_x3(&tx[i], c.x, (uint64_t)a.rows, (uint64_t)a.K, 32u << i)) return TRB_ERR_CUDA;
+  if (!make_map_2d(&tq, CU_TENSOR_MAP_DATA_TYPE_INT32, 4, c.q, (uint64_t)c.num_deltas * slabs, 2ull * a.N, Cfg::SLABS, 256,
                    CU_TENSOR_MAP_SWIZZLE_NONE))
     return TRB_ERR_CUDA;
-  if (!make_map_2d(&tm, CU_TENSOR_MAP_DATA_TYPE_INT32, 4, c.meta, (uint64_t)c.num_deltas * slabs, (uint64_t)a.N, 2, 128,
-                   CU_TENSOR_MAP_SWIZZLE_NONE))
+  if (!make_map_2d(&tm, CU_TENSOR_MAP_DATA_TYPE_INT32, 4, c.meta, (uint64_t)c.num_deltas * slabs, (uint64_t)a.N, Cfg::SLABS,
+                   128, CU_TENSOR_MAP_SWIZZLE_NONE))
     return TRB_ERR_CUDA;
   if (a.grouped) {
     if (!make_map_2d(&ts, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, c.s, (uint64_t)c.num_deltas * groups, (uint64_t)a.N, 1, 128,
@@ -137,12 +152,12 @@ static int launch_tc_impl(Kernel kernel, const GemmCall& c, const GemmArgs& a) {
   } else {
     ts = tm;  // never dereferenced
   }
-  static std::atomic<bool> attr_set[64];   // one per instantiation of this template, that is per kernel
-  if (!ensure_smem_attr(kernel, c.dev, Cfg::SMEM_ALLOC, attr_set)) return TRB_ERR_CUDA;
+  static std::atomic<bool> attr_set[64];
+  if (!ensure_smem_attr(delta_gemm_tcsp_kernel, c.dev, Cfg::SMEM_ALLOC, attr_set)) return TRB_ERR_CUDA;
   constexpr int ctas = Cfg::CTAS;
   int grid = sm_count(c.dev);
   if (c.sms > 0 && c.sms < grid) grid = c.sms;
-  grid /= ctas;                      // work items go to CTAs, or to clusters of two
+  grid /= ctas;                      // work items go to clusters of two
   if (grid < 1) grid = 1;
   const int n_stripes = (a.N + Cfg::SW * 64 - 1) / (Cfg::SW * 64);
   long long max_tiles;
@@ -166,14 +181,10 @@ static int launch_tc_impl(Kernel kernel, const GemmCall& c, const GemmArgs& a) {
   at[1].val.programmaticStreamSerializationAllowed = 1;
   lc.attrs = at;
   lc.numAttrs = 2;
-  return cudaLaunchKernelEx(&lc, kernel, tx, tq, tm, ts, a) == cudaSuccess ? TRB_OK : TRB_ERR_CUDA;
+  return cudaLaunchKernelEx(&lc, delta_gemm_tcsp_kernel, tx[0], tx[1], tx[2], tq, tm, ts, a) == cudaSuccess ? TRB_OK
+                                                                                                            : TRB_ERR_CUDA;
 }
-static int launch_tc(const GemmCall& c, const GemmArgs& a) {
-  // The sparse kernel writes y in 16-byte pieces of 8 output features.
-  if ((reinterpret_cast<uintptr_t>(a.y) & 15) != 0 || (a.N & 7) != 0) return TRB_ERR_KERN_SHAPE;
-  return launch_tc_impl<TcSpPairCfg>(delta_gemm_tcsp_kernel<true>, c, a);
-}
-static_assert(TcSpPairCfg::SMEM_ALLOC <= 232448, "shared memory budget of one sm_100 CTA");
+static_assert(TcSpCfg::SMEM_ALLOC <= 232448, "shared memory budget of one sm_100 CTA");
 
 // The mma.sp kernel works on tiles of 8 tokens (decode: a delta has a handful of tokens).  Larger
 // tile classes of the same kernel (16 and 32 tokens) were built and measured: compiled beside the

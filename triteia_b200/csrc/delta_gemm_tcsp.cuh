@@ -1,34 +1,40 @@
 // Grouped 2:4-sparse int4 delta GEMM for prefill-sized token tiles on the SPARSE fifth-generation
 // tensor-core instruction: tcgen05.mma.sp (kind::f16, K = 32 dense per instruction), A operand = the
-// STORED halves of the 2:4 weights in shared memory (16 per row and instruction), 2:4 metadata in
-// tensor memory, fp32 accumulator in tensor memory.
+// STORED halves of the 2:4 weights and their 2:4 metadata, both in tensor memory, B operand = the
+// activation tile in shared memory, fp32 accumulator in tensor memory.
 //
-// Forms of the kernel template:
-//   PAIR (shipped)  two CTAs of a cluster issue one tcgen05.mma.sp.cta_group::2 per instruction:
-//                   M = 256 output features (128 per CTA: each CTA decodes its own stripe and holds its
-//                   own accumulator and metadata) x N = 256 tokens (each CTA stages 128 of them).  The
-//                   leader CTA's MMA thread issues for both; every decode warp of both CTAs arrives on
-//                   the leader's barrier; tcgen05.commit with a CTA mask hands stages back to both.
-//                   Half the activation bytes per SM and flop: the kernel is bound by what one SM can
-//                   pull through TMA and shared memory, not by the tensor pipe.
-//   single CTA      M = 128 x N = 256 per CTA (PAIR = false; not instantiated in the library).
+// Two CTAs of a cluster issue one tcgen05.mma.sp.cta_group::2 per instruction: M = 256 output features
+// (128 per CTA: each CTA decodes its own stripe and holds its own accumulator, weights and metadata) x
+// N = 64, 128 or 256 tokens, the smallest that holds the tile (each CTA stages half of them).  The
+// leader CTA's MMA thread issues for both; every decode warp of both CTAs arrives on the leader's
+// barrier; tcgen05.commit with a CTA mask hands stages back to both.
 //
-// Per 64-K chunk and per CTA:
-//   producer warps  TMA, one thread each: the activation tile [tokens x 64 K] (128-byte swizzle, the B
-//                   operand as it lands) / packed weights + metadata + scales of the CTA's 128 columns
-//   16 decode warps two teams of eight on alternate chunks: nibbles -> fp16 (x group scale) stored as
-//                   half2 pairs into the compressed A tile [128 features x 32 stored halves] (64-byte
-//                   swizzle, K-major); the same warps copy the chunk's metadata into TMEM with
-//                   tcgen05.st: the packed format already holds, per 32-K slab, one 16-bit field per
-//                   row and K half in the tensor core's ordered 2-bit-index form, so a TMEM cell
-//                   (lane = 16*(row/16) + 8*(K half) + row%8) is two such fields (rows r and r + 8)
-//                   picked from two packed words with one PRMT
-//   MMA warp        one thread issues 2 tcgen05.mma.sp per chunk; the metadata operand is the even
-//                   column of the chunk's column pair, the instruction descriptor's id2 selects the
-//                   slab; tcgen05.commit hands the stage back / publishes the tile
-//   4 epilogue warps tcgen05.ld, scale, convert, transpose 32 x 32 blocks through shared memory and
+// Per 128-K chunk (one scale group, four instructions) and per CTA:
+//   producer warps  TMA, one thread each: the activation tile [tokens x 128 K] as two 128-byte-swizzled
+//                   halves in one 3-D box (the B operand as it lands) / packed weights, metadata and
+//                   scales of the CTA's 128 columns
+//   12 decode warps three teams of four (one warp per TMEM lane quadrant) on alternate chunks; a lane owns
+//                   one feature: its nibbles -> fp16 (x group scale) -> tcgen05.st into the A columns of
+//                   the stage, 8 columns per 32-K slab, and its metadata cells.  The packed format already
+//                   holds, per slab, one 16-bit field per row and K half in the tensor core's ordered
+//                   2-bit-index form, so a metadata cell (lane = 16*(row/16) + 8*(K half) + row%8) is two
+//                   such fields (rows r and r + 8) picked from two packed words with one PRMT
+//   MMA warp        one thread issues 4 tcgen05.mma.sp per chunk; a slab's metadata is one column of a
+//                   pair, the instruction descriptor's id2 selects it; tcgen05.commit hands the stage back
+//   8 epilogue warps tcgen05.ld, scale, convert, transpose 32 x 32 blocks through shared memory and
 //                   store 16-byte pieces (8 features of one token)
-// TMEM: columns [0, 256) accumulator, [256, 256 + 2 * stages) metadata (a column pair per stage).
+// TMEM: columns [0, 256) accumulator (one of 256 tokens, or two of up to 128 in turn, so that the
+// epilogue of a small tile overlaps the next one's chunks), then 32 columns of weights and 4 of metadata
+// per stage.
+//
+// What bounds it: the 128 B/clk shared-memory pipe of an SM.  Per 64 K a 256-token tile needs 128
+// wavefronts for the activations landing, 128 for the tensor core reading them, 25 for the packed
+// weights and about 50 for their decode, against 247 cycles of the instruction.  Weights in shared memory
+// would add 64 for the decode's stores and 64 for the tensor core, and a proxy fence on the decode
+// warps' chain.
+// Measured, whole calls (before: weights through shared memory, 64-K stages, every tile as 256 tokens, one
+// accumulator): 8192 tokens in 16 segments, 5120 -> 13824: 857 -> 721 us; 1531 tokens, one weight, 4096 -> 11008:
+// 109 -> 91 us; 700 tokens over 13 deltas (54 each), 4096 -> 12288: 229 -> 127 us.
 // Every wait is bounded; both CTAs of a pair meet at a cluster barrier before either leaves.
 #pragma once
 
@@ -36,29 +42,23 @@
 
 namespace trb {
 
-// PAIR: two CTAs of a cluster share one tcgen05.mma.sp.cta_group::2 (M = 256 features, 128 per CTA;
-// each CTA stages half of the token tile), which halves the activation bytes every SM pulls through
-// its shared memory per flop.
-template <bool PAIR_>
-struct TcSpCfgT {
-  static constexpr bool PAIR = PAIR_;
-  static constexpr int CTAS = PAIR ? 2 : 1;
-  static constexpr int TT = 256;
-  static constexpr int SW = 2 * CTAS;       // 64-column blocks per work item (128 columns per CTA)
-  static constexpr int KC = 64;             // dense K per stage = two sparse MMAs
-  static constexpr int STAGES = PAIR ? 6 : 4;
-  static constexpr int B_ROWS = TT / CTAS;  // tokens of the tile staged by one CTA
-  static constexpr int DECODE_TEAMS = 2;    // teams of 8 warps take alternate K chunks
-  static constexpr int DECODE_WARPS = 8 * DECODE_TEAMS;
-  static constexpr int EPI_WARPS = 8;       // two per TMEM lane quadrant: each drains half of the token batches
-  static constexpr int THREADS = (3 + DECODE_WARPS + EPI_WARPS) * 32;
-  static constexpr int A_BYTES = 128 * (KC / 2) * 2;     // 8 KiB of stored halves
-  static constexpr int B_BYTES = B_ROWS * KC * 2;        // 32 KiB, 16 KiB per CTA of a pair
-  static constexpr int Q_BYTES = 2 * 256 * 4;
-  static constexpr int M_BYTES = 2 * 128 * 4;
+struct TcSpCfg {
+  static constexpr int CTAS = 2;            // CTAs of a cluster that share a work item
+  static constexpr int TT = 256;            // largest token tile
+  static constexpr int SW = 4;              // 64-column blocks per work item (128 columns per CTA)
+  static constexpr int KC = 128;            // dense K per stage: one scale group, four sparse MMAs
+  static constexpr int SLABS = KC / 32;
+  static constexpr int STAGES = 5;
+  static constexpr int TEAMS = 3;           // teams of 4 decode warps take alternate chunks
+  static constexpr int DECODE0 = 4;         // warps 0-2: activation TMA, MMA, weight TMA; 3 idle (quadrants start at a multiple of 4)
+  static constexpr int EPI0 = DECODE0 + 4 * TEAMS;
+  static constexpr int EPI_WARPS = 8;       // two per TMEM lane quadrant
+  static constexpr int THREADS = (EPI0 + EPI_WARPS) * 32;
+  static constexpr int B_BYTES = (TT / CTAS) * KC * 2;   // 32 KiB per CTA at 256 tokens
+  static constexpr int Q_BYTES = SLABS * 256 * 4;
+  static constexpr int M_BYTES = SLABS * 128 * 4;
   static constexpr int S_BYTES = 256;
-  static constexpr int A_OFF = 0;
-  static constexpr int B_OFF = A_OFF + A_BYTES;
+  static constexpr int B_OFF = 0;
   static constexpr int Q_OFF = B_OFF + B_BYTES;
   static constexpr int M_OFF = Q_OFF + Q_BYTES;
   static constexpr int S_OFF = M_OFF + M_BYTES;
@@ -67,46 +67,42 @@ struct TcSpCfgT {
   static constexpr int XPOSE_OFF = ROWS_OFF + TT * 4;                     // [EPI_WARPS][32 tokens][32 features] halves
   static constexpr int PREFIX_OFF = XPOSE_OFF + EPI_WARPS * 2048;
   static constexpr int BAR_OFF = PREFIX_OFF + (kMaxSegments + 2) * 4;
-  static constexpr int NUM_BARS = 3 * STAGES + 2;
+  static constexpr int NUM_BARS = 3 * STAGES + 4;
   static constexpr int SMEM_BYTES = BAR_OFF + NUM_BARS * 8 + 16;
   static constexpr int SMEM_ALLOC = SMEM_BYTES + 1024;
   static constexpr uint32_t TMEM_COLS = 512;
-  static constexpr uint32_t META_COL = 256;             // even: column pairs start on even columns
+  static constexpr uint32_t A_COL = 256;                       // weights of stage st: columns A_COL + 32 * st, 8 per slab
+  static constexpr uint32_t META_COL = A_COL + 32 * STAGES;    // metadata of stage st: META_COL + 4 * st, a column per slab
+  static_assert(META_COL % 2 == 0 && META_COL + 4 * STAGES <= TMEM_COLS, "metadata pairs start on even columns");
 };
-using TcSpCfg = TcSpCfgT<false>;
-using TcSpPairCfg = TcSpCfgT<true>;
 
-// K-major, 64-byte swizzle: rows of 64 bytes, 8-row groups 512 bytes apart, layout type 4.
-__device__ __forceinline__ uint64_t tc_smem_desc_sw64(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr >> 4) & 0x3FFF);
-  d |= (uint64_t)1 << 16;
-  d |= (uint64_t)(512 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)4 << 61;
-  return d;
-}
+// Token tile class of a work item: N of the instruction = 64 << class.
+__device__ __forceinline__ int tile_class(int valid) { return valid <= 64 ? 0 : (valid <= 128 ? 1 : 2); }
 
-// Sparse kind::f16: the dense descriptor plus the sparsity flag (bit 2) and the metadata id (bits 0-1).
-__device__ __forceinline__ void tc_mma_sp_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t e_tmem,
-                                              uint32_t id2, uint32_t accumulate) {
-  const uint32_t idesc = kTcIdesc | (1u << 2) | (id2 & 3u);
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.sp.cta_group::1.kind::f16 [%0], %1, %2, [%9], %3, {%5, %6, %7, %8}, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u),
-        "r"(e_tmem)
-      : "memory");
-}
-
-__device__ __forceinline__ void tc_st1(uint32_t taddr, uint32_t v) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(taddr), "r"(v) : "memory");
-}
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-__device__ __forceinline__ void sts32(uint32_t addr, uint32_t v) {
-  asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+__device__ __forceinline__ void tc_st4(uint32_t taddr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(a), "r"(b), "r"(c), "r"(d)
+               : "memory");
+}
+__device__ __forceinline__ void tc_st8(uint32_t taddr, const uint32_t (&v)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(v[0]), "r"(v[1]),
+               "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
+}
+// 3-D tiled TMA load of the activation tile: coordinates (K inside a 64-K half, row, 64-K half).
+__device__ __forceinline__ void tma_load_3d_hint(void* dst, const CUtensorMap* map, int c0, int c1, int c2, uint64_t* bar,
+                                                 uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint "
+      "[%0], [%1, {%2, %3, %4}], [%5], %6;" ::"r"(smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar)), "l"(policy)
+      : "memory");
+}
+__device__ __forceinline__ uint32_t lds16(uint32_t addr) {
+  uint16_t v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr) : "memory");
+  return v;
 }
 
 // ---- cluster-of-two helpers ----
@@ -151,17 +147,16 @@ __device__ __forceinline__ void mbar_wait_cluster(uint64_t* bar, uint32_t parity
     }
   }
 }
-// One instruction for both CTAs: M = 256 (128 TMEM lanes in each CTA), N = 256 tokens (128 rows of B
-// from each CTA's shared memory), descriptors and TMEM addresses are CTA-relative and equal in both.
-__device__ __forceinline__ void tc_mma_sp_f16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t e_tmem,
-                                                   uint32_t id2, uint32_t accumulate) {
-  constexpr uint32_t kIdesc = (1u << 4) | ((256u >> 3) << 17) | ((256u >> 4) << 24) | (1u << 2);
-  const uint32_t idesc = kIdesc | (id2 & 3u);
+// One instruction for both CTAs: M = 256 (128 TMEM lanes in each CTA), half of the N tokens from each
+// CTA's shared memory; TMEM addresses and the descriptor are CTA-relative and equal in both.
+// `idesc`: D fp32, A and B fp16, K-major, M = 256, N, the sparsity flag (bit 2) and the metadata id (bits 0-1).
+__device__ __forceinline__ void tc_mma_sp_f16_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t e_tmem,
+                                                   uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.sp.cta_group::2.kind::f16 [%0], %1, %2, [%6], %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u), "r"(e_tmem)
+      "tcgen05.mma.sp.cta_group::2.kind::f16 [%0], [%1], %2, [%6], %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u), "r"(e_tmem)
       : "memory");
 }
 // Arrive on the barrier at this shared-memory offset in both CTAs once the pair's MMAs issued so far retire.
@@ -171,23 +166,23 @@ __device__ __forceinline__ void tc_commit_pair(uint64_t* bar) {
                : "memory");
 }
 
-template <bool PAIR>
-__global__ void __launch_bounds__(TcSpCfgT<PAIR>::THREADS, 1)
-delta_gemm_tcsp_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_q,
+__global__ void __launch_bounds__(TcSpCfg::THREADS, 1)
+delta_gemm_tcsp_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_constant__ CUtensorMap tm_x1,
+                       const __grid_constant__ CUtensorMap tm_x2, const __grid_constant__ CUtensorMap tm_q,
                        const __grid_constant__ CUtensorMap tm_m, const __grid_constant__ CUtensorMap tm_s,
-                       const GemmArgs a) {
-  using Cfg = TcSpCfgT<PAIR>;
+                       const __grid_constant__ GemmArgs a) {
+  using Cfg = TcSpCfg;
   constexpr int STAGES = Cfg::STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   int* rows = reinterpret_cast<int*>(smem + Cfg::ROWS_OFF);
   int* prefix = reinterpret_cast<int*>(smem + Cfg::PREFIX_OFF);
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + Cfg::BAR_OFF);   // TMA data of a stage landed
-  uint64_t* aready_bar = full_bar + STAGES;                                // A tile + metadata of a stage written
+  uint64_t* aready_bar = full_bar + STAGES;                                // leader: weights + metadata of a stage in TMEM, both CTAs
   uint64_t* empty_bar = aready_bar + STAGES;                               // MMAs of a stage retired
-  uint64_t* accready_bar = empty_bar + STAGES;                             // accumulator complete
-  uint64_t* accfree_bar = accready_bar + 1;                                // accumulator drained
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accfree_bar + 1);
+  uint64_t* accready_bar = empty_bar + STAGES;                             // [2] accumulator complete
+  uint64_t* accfree_bar = accready_bar + 2;                                // [2] leader: accumulator half drained by both CTAs
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accfree_bar + 2);
   volatile int* dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x;
@@ -207,26 +202,21 @@ delta_gemm_tcsp_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
   if (tid == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full_bar[s], 1);
-      mbar_init(&aready_bar[s], 8 * Cfg::CTAS);   // pair: the leader's barrier counts both CTAs' warps
+      mbar_init(&aready_bar[s], 4 * Cfg::CTAS);   // the leader's barrier counts both CTAs' warps of a team
       mbar_init(&empty_bar[s], 1);
     }
-    mbar_init(accready_bar, 1);
-    mbar_init(accfree_bar, Cfg::EPI_WARPS * Cfg::CTAS);
+    for (int h = 0; h < 2; ++h) {
+      mbar_init(&accready_bar[h], 1);
+      mbar_init(&accfree_bar[h], Cfg::EPI_WARPS * Cfg::CTAS);
+    }
     *dead = 0;
     fence_mbar_init();
   }
   if (warp == 1) {
-    if constexpr (PAIR) {
-      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                   "r"(Cfg::TMEM_COLS)
-                   : "memory");
-      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-    } else {
-      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                   "r"(Cfg::TMEM_COLS)
-                   : "memory");
-      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"(Cfg::TMEM_COLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   pdl_wait();   // everything below reads what the kernels launched before this one wrote
   n_seg = a.n_seg_ptr ? *a.n_seg_ptr : a.n_seg;
@@ -256,7 +246,7 @@ delta_gemm_tcsp_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
   }
   tc_fence_before();
   __syncthreads();
-  if constexpr (PAIR) cluster_sync_all();     // both CTAs' barriers exist before any remote arrive
+  cluster_sync_all();     // both CTAs' barriers exist before any remote arrive
   tc_fence_after();
   if (a.mode == kSegList) total_tiles = prefix[n_seg];
   else total_tiles = a.mode == kSegTiles ? n_seg : (a.mode == kSegSingle ? (a.rows + Cfg::TT - 1) / Cfg::TT : a.rows);
@@ -264,37 +254,38 @@ delta_gemm_tcsp_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
 
   const int n_stripes = (a.N + Cfg::SW * 64 - 1) / (Cfg::SW * 64);
   const int n_items = total_tiles * n_stripes;
-  // Work items go round-robin over CTAs, or over CTA pairs: CTA `rank` of a pair owns columns
-  // [col0 + 128 * rank, +128) of the item and stages tokens [row0 + 128 * rank, +128) of its tile.
-  const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
-  const int item0 = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
-  const int item_step = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
+  // Work items go round-robin over CTA pairs: CTA `rank` of a pair owns columns [col0 + 128 * rank, +128)
+  // of the item and stages its half of the tile's tokens.
+  const uint32_t rank = cluster_ctarank();
+  const int item0 = (int)(blockIdx.x >> 1);
+  const int item_step = (int)(gridDim.x >> 1);
   const int my_col = (int)rank * 128;
   const int slabs = a.K / 32;
-  const int k_chunks = a.K / Cfg::KC;
-  const int groups = a.grouped ? a.K / 128 : 1;
+  const int k_chunks = a.K / Cfg::KC;      // K is a multiple of 128
   const uint32_t smem_base = smem_u32(smem);
 
   if (warp == 0) {
     // ------------------------------ TMA producer: activations ------------------------------
     if (lane == 0) {
-      prefetch_tmap(&tm_x);
-      prefetch_tmap(&tm_q);
-      prefetch_tmap(&tm_m);
-      if (a.grouped) prefetch_tmap(&tm_s);
+      prefetch_tmap(&tm_x0);
+      prefetch_tmap(&tm_x1);
+      prefetch_tmap(&tm_x2);
       const uint64_t pol_x = policy_evict_last();
-      const uint32_t stage_tx = Cfg::B_BYTES + Cfg::Q_BYTES + Cfg::M_BYTES + (a.grouped ? Cfg::S_BYTES : 0);
       int st = 0;
       uint32_t phase = 0;
       for (int item = item0; item < n_items; item += item_step) {
-        WorkItem w = decode_item<Cfg>(a, prefix, n_seg, n_stripes, item);
+        const WorkItem w = decode_item<Cfg>(a, prefix, n_seg, n_stripes, item);
         if (!w.ok) continue;
+        const int cls = tile_class(w.valid);
+        const int half = 32 << cls;            // rows of the tile staged by this CTA
+        const CUtensorMap* tm_x = cls == 0 ? &tm_x0 : (cls == 1 ? &tm_x1 : &tm_x2);
+        const uint32_t stage_tx = half * Cfg::KC * 2 + Cfg::Q_BYTES + Cfg::M_BYTES + (a.grouped ? Cfg::S_BYTES : 0);
+        const int row0 = w.row0 + (int)rank * half;
         for (int kc = 0; kc < k_chunks; ++kc) {
           mbar_wait(&empty_bar[st], phase ^ 1, dead);
-          uint8_t* sbase = smem + st * Cfg::STAGE_BYTES;
           // The stage's one arrival, carrying the bytes of this load and of the weight producer's loads.
           mbar_arrive_expect_tx(&full_bar[st], stage_tx);
-          tma_load_2d_hint(sbase + Cfg::B_OFF, &tm_x, kc * Cfg::KC, w.row0 + (int)rank * Cfg::B_ROWS, &full_bar[st], pol_x);
+          tma_load_3d_hint(smem + st * Cfg::STAGE_BYTES + Cfg::B_OFF, tm_x, 0, row0, 2 * kc, &full_bar[st], pol_x);
           if (++st == STAGES) { st = 0; phase ^= 1; }
         }
       }
@@ -303,156 +294,157 @@ delta_gemm_tcsp_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
     // ------------------------------ MMA issuer ------------------------------
     if (lane == 0 && rank == 0) {
       int st = 0;
-      uint32_t phase = 0, use = 0;
+      uint32_t phase = 0, used[2] = {0, 0};
+      int turn = 0;
       for (int item = item0; item < n_items; item += item_step) {
-        WorkItem w = decode_item<Cfg>(a, prefix, n_seg, n_stripes, item);
-        w.col0 += my_col;
+        const WorkItem w = decode_item<Cfg>(a, prefix, n_seg, n_stripes, item);
         if (!w.ok) continue;
-        if constexpr (PAIR) mbar_wait_cluster(accfree_bar, (use & 1) ^ 1, dead);
-        else mbar_wait(accfree_bar, (use & 1) ^ 1, dead);
+        const int cls = tile_class(w.valid);
+        // A 256-token tile takes both halves of the accumulator columns, smaller ones take turns.
+        const int h = cls == 2 ? 0 : turn;
+        mbar_wait_cluster(&accfree_bar[h], (used[h] & 1) ^ 1, dead);
+        ++used[h];
+        if (cls == 2) {
+          mbar_wait_cluster(&accfree_bar[1], (used[1] & 1) ^ 1, dead);
+          ++used[1];
+        } else {
+          turn ^= 1;
+        }
         tc_fence_after();
+        const uint32_t d_tmem = tmem_base + h * 128;
+        const uint32_t idesc = (1u << 4) | ((uint32_t)(8 << cls) << 17) | ((256u >> 4) << 24) | (1u << 2);   // N = 64 << cls
+        const uint32_t khalf = (32u << cls) * 128u >> 4;      // descriptor step to the second 64-K half
         for (int kc = 0; kc < k_chunks; ++kc) {
-          if constexpr (PAIR) {
-            // Every decode warp of both CTAs arrives after its own CTA's TMA data landed and its part of
-            // the A tile and metadata is written: the one barrier covers both CTAs' operands.
-            mbar_wait_cluster(&aready_bar[st], phase, dead);
-          } else {
-            mbar_wait(&full_bar[st], phase, dead);
-            mbar_wait(&aready_bar[st], phase, dead);
-          }
+          // Every decode warp of both CTAs arrives after its own CTA's TMA data landed and its part of
+          // the weights and metadata is in TMEM: the one barrier covers both CTAs' operands.
+          mbar_wait_cluster(&aready_bar[st], phase, dead);
           tc_fence_after();
-          const uint32_t sb = smem_base + st * Cfg::STAGE_BYTES;
-          const uint64_t adesc = tc_smem_desc_sw64(sb + Cfg::A_OFF);
-          const uint64_t bdesc = tc_smem_desc(sb + Cfg::B_OFF);
-          const uint32_t e_tmem = tmem_base + Cfg::META_COL + 2 * st;
+          const uint64_t bdesc = tc_smem_desc(smem_base + st * Cfg::STAGE_BYTES + Cfg::B_OFF);
+          const uint32_t a_tmem = tmem_base + Cfg::A_COL + 32 * st;
+          const uint32_t e_tmem = tmem_base + Cfg::META_COL + 4 * st;
 #pragma unroll
-          for (int k = 0; k < 2; ++k) {  // per instruction: 32 bytes of stored A, 64 bytes of B, metadata column k of the pair
-            if constexpr (PAIR) tc_mma_sp_f16_pair(tmem_base, adesc + 2 * k, bdesc + 4 * k, e_tmem, k, (kc > 0 || k > 0) ? 1u : 0u);
-            else tc_mma_sp_f16(tmem_base, adesc + 2 * k, bdesc + 4 * k, e_tmem, k, (kc > 0 || k > 0) ? 1u : 0u);
-          }
-          if constexpr (PAIR) tc_commit_pair(&empty_bar[st]);
-          else tc_commit(&empty_bar[st]);
+          for (int k = 0; k < Cfg::SLABS; ++k)   // per instruction: 8 columns of weights, 64 bytes of B, one metadata column
+            tc_mma_sp_f16_pair(d_tmem, a_tmem + 8 * k, bdesc + (k >> 1) * khalf + 4 * (k & 1), e_tmem + (k & 2),
+                               idesc | (k & 1), (kc > 0 || k > 0) ? 1u : 0u);
+          tc_commit_pair(&empty_bar[st]);
           if (++st == STAGES) { st = 0; phase ^= 1; }
         }
-        if constexpr (PAIR) tc_commit_pair(accready_bar);
-        else tc_commit(accready_bar);
-        ++use;
+        tc_commit_pair(&accready_bar[h]);
       }
     }
-  } else if (warp < 2 + Cfg::DECODE_WARPS) {
-    // ------------------------------ decode warps: packed -> compressed A tile + metadata ------------------------------
-    // Warp dw handles column block cb = dw / 4 and row groups g = 2 * (dw % 4) + u; lane bits are
-    // (j high, slab s, lane-in-quad m, j low): it decodes weight word (s, cb, g, m, j) for u = 0, 1.
-    const int team = (warp - 2) >> 3;
-    const int dw = (warp - 2) & 7;
-    const int cb = dw >> 2;
-    const int s = (lane >> 3) & 1, m = (lane >> 1) & 3, j = ((lane >> 4) << 1) | (lane & 1);
-    uint32_t q_off[2], s_off[2], st_off[2][4];
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int g = 2 * (dw & 3) + u;
-      q_off[u] = Cfg::Q_OFF + s * 1024 + cb * 512 + (4 * g + m) * 16 + j * 4;
-      s_off[u] = Cfg::S_OFF + (cb * 64 + 8 * g + 2 * j) * 2;
-      const int n0 = cb * 64 + 8 * g + j;            // block-0 row; block-1 row is n0 + 4
-#pragma unroll
-      for (int p = 0; p < 4; ++p) {                  // pairs: (n0, grp m), (n0, grp m+4), (n1, m), (n1, m+4)
-        const int n = n0 + 4 * (p >> 1);
-        const int kc4 = 8 * s + m + 4 * (p & 1);     // 4-byte pair index inside the 64-byte row (= K group of the chunk)
-        st_off[u][p] = Cfg::A_OFF + (n >> 3) * 512 + (n & 7) * 64 + ((((kc4 >> 2) ^ ((n >> 1) & 3))) << 4) + (kc4 & 3) * 4;
-      }
-    }
-    // Metadata duty: TMEM lanes of this warp's quadrant, slab ms of the chunk.  Lane L of the tile is
-    // (row block L / 16, K half (L / 8) % 2, row L % 8): its cell is the 16-bit field of that K half for
-    // rows r = 16 * (L / 16) + L % 8 (low) and r + 8 (high).  Row r of the stripe is column block r / 64,
-    // group g = (r % 64) / 8, position r % 8 = j + 4 * hi: its field is the low (hi = 0) or high half of
-    // metadata word 2 * (j & 1) + 32 * (j >> 1) + 4 * g + (K half) of that block; r + 8 is group g + 1.
-    const int quad = warp & 3;
-    const int ms = dw >> 2;
-    const int L = quad * 32 + lane;
-    const int mr = 16 * (L >> 4) + (L & 7);
-    const int mk1 = (L >> 3) & 1;
-    const int mj = mr & 3, mhi = (mr >> 2) & 1, mg = (mr & 63) >> 3;
-    const uint32_t ma_off = Cfg::M_OFF + ms * 512 + ((mr >> 6) * 64 + 2 * (mj & 1) + 32 * (mj >> 1) + 4 * mg + mk1) * 4;
-    const uint32_t msel = mhi ? 0x7632u : 0x5410u;
-    const uint32_t e_lane = tmem_base + ((uint32_t)(quad * 32) << 16) + Cfg::META_COL + ms;
-
-    const uint32_t aready_leader = PAIR ? mapa_shared(smem_u32(aready_bar), 0) : 0u;
-    int st = 0;
-    uint32_t phase = 0, chunk = 0;
-    for (int item = item0; item < n_items; item += item_step) {
-      WorkItem w = decode_item<Cfg>(a, prefix, n_seg, n_stripes, item);
-      w.col0 += my_col;
-      if (!w.ok) continue;
-      for (int kc = 0; kc < k_chunks; ++kc, ++chunk) {
-        if ((int)(chunk % Cfg::DECODE_TEAMS) != team) {     // the other team's chunk
-          if (++st == STAGES) { st = 0; phase ^= 1; }
-          continue;
-        }
-        if (dw == 0) mbar_wait(&full_bar[st], phase, dead);   // one warp of the team polls
-        named_bar_sync(5 + team, 256);
-        const uint32_t sb = smem_base + st * Cfg::STAGE_BYTES;
-        {
-          const uint32_t wa = lds32(sb + ma_off), wb = lds32(sb + ma_off + 16);
-          tc_st1(e_lane + 2 * st, __byte_perm(wa, wb, msel));
-        }
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const uint32_t q = lds32(sb + q_off[u]);
-          uint32_t v[4];
-          int4x4_to_half2x2(q, v[0], v[1]);
-          int4x4_to_half2x2(q >> 8, v[2], v[3]);
-          if (a.grouped) {
-            const uint32_t sc = lds32(sb + s_off[u]);  // (scale of n0, scale of n1)
-            const uint32_t s0 = __byte_perm(sc, 0, 0x1010), s1 = __byte_perm(sc, 0, 0x3232);
-            v[0] = hmul2_u32(v[0], s0); v[1] = hmul2_u32(v[1], s0);
-            v[2] = hmul2_u32(v[2], s1); v[3] = hmul2_u32(v[3], s1);
-          }
-#pragma unroll
-          for (int p = 0; p < 4; ++p) sts32(sb + st_off[u][p], v[p]);
-        }
-        tc_wait_st();
-        fence_proxy_async();      // the tensor core reads the A tile through the async proxy
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) {
-          if constexpr (PAIR) mbar_arrive_cluster(aready_leader + st * 8);
-          else mbar_arrive(&aready_bar[st]);
-        }
-        if (++st == STAGES) { st = 0; phase ^= 1; }
-      }
-    }
-  } else if (warp == 2 + Cfg::DECODE_WARPS + Cfg::EPI_WARPS) {
+  } else if (warp == 2) {
     // ------------------------------ TMA producer: packed weights, metadata, scales ------------------------------
     // A thread of its own: the TMA unit takes the small boxes while the activation box is in flight.
     if (lane == 0) {
+      prefetch_tmap(&tm_q);
+      prefetch_tmap(&tm_m);
+      if (a.grouped) prefetch_tmap(&tm_s);
       const uint64_t pol_w = policy_evict_first();
       int st = 0;
       uint32_t phase = 0;
       for (int item = item0; item < n_items; item += item_step) {
-        WorkItem w = decode_item<Cfg>(a, prefix, n_seg, n_stripes, item);
-        w.col0 += my_col;
+        const WorkItem w = decode_item<Cfg>(a, prefix, n_seg, n_stripes, item);
         if (!w.ok) continue;
+        const int col0 = w.col0 + my_col;
         for (int kc = 0; kc < k_chunks; ++kc) {
           mbar_wait(&empty_bar[st], phase ^ 1, dead);
           uint8_t* sbase = smem + st * Cfg::STAGE_BYTES;
-          const int wrow = w.delta * slabs + kc * 2;
-          tma_load_2d_hint(sbase + Cfg::Q_OFF, &tm_q, (w.col0 / 64) * 128, wrow, &full_bar[st], pol_w);
-          tma_load_2d_hint(sbase + Cfg::M_OFF, &tm_m, (w.col0 / 64) * 64, wrow, &full_bar[st], pol_w);
+          const int wrow = w.delta * slabs + kc * Cfg::SLABS;
+          tma_load_2d_hint(sbase + Cfg::Q_OFF, &tm_q, (col0 / 64) * 128, wrow, &full_bar[st], pol_w);
+          tma_load_2d_hint(sbase + Cfg::M_OFF, &tm_m, (col0 / 64) * 64, wrow, &full_bar[st], pol_w);
           if (a.grouped)
-            tma_load_2d_hint(sbase + Cfg::S_OFF, &tm_s, w.col0, w.delta * groups + kc / 2, &full_bar[st], pol_w);
+            tma_load_2d_hint(sbase + Cfg::S_OFF, &tm_s, col0, w.delta * k_chunks + kc, &full_bar[st], pol_w);
           if (++st == STAGES) { st = 0; phase ^= 1; }
         }
       }
     }
-  } else {
-    // ------------------------------ epilogue warps ------------------------------
-    const int ew = warp - 2 - Cfg::DECODE_WARPS;
+  } else if (warp >= Cfg::DECODE0 && warp < Cfg::EPI0) {
+    // ------------------------------ decode warps: packed -> weights + metadata in TMEM ------------------------------
+    // Lane of quadrant `quad` = feature n = 32 * quad + lane of the CTA's 128: column block cb = n / 64, group
+    // g = n / 8 % 8, position j + 4 * hi inside the group.  Its stored pairs m and m + 4 (m = 0..3) of a slab
+    // are the low (hi = 0) or the odd (hi = 1) byte pair of weight word (slab, cb, g, m, j).
+    const int team = (warp - Cfg::DECODE0) >> 2;
     const int quad = warp & 3;
-    uint32_t use = 0;
+    const int n = quad * 32 + lane;
+    const int j = lane & 3, hi = (lane >> 2) & 1, g = (n >> 3) & 7;
+    // Groups g and g + 2 lie on the same banks: half of the lanes read the words of a pair in the other order.
+    const bool flip = (g & 2) != 0;
+    const uint32_t q_off = Cfg::Q_OFF + (n >> 6) * 512 + g * 64 + j * 4;
+    const uint32_t q_first = q_off + (flip ? 16 : 0), q_second = q_off + (flip ? 0 : 16);
+    const uint32_t s_off = Cfg::S_OFF + ((n & ~7) + 2 * j + hi) * 2;     // stored scale order inside 8 columns: 0 4 1 5 2 6 3 7
+    const int shift = 8 * hi;
+    // Metadata cell of TMEM lane n: (row block n / 16, K half n / 8 % 2, row n % 8) = the 16-bit field of that K
+    // half for rows r = 16 * (n / 16) + n % 8 (low) and r + 8 (high).  Row r is block r / 64, group mg, position
+    // mj + 4 * mhi: its field is the low (mhi = 0) or high half of metadata word
+    // 2 * (mj & 1) + 32 * (mj >> 1) + 4 * mg + (K half) of that block; r + 8 is group mg + 1.  Lanes with
+    // mj >= 2 fetch the two words in the other order (same banks otherwise).
+    const int mr = 16 * (n >> 4) + (n & 7);
+    const int mj = mr & 3, mhi = (mr >> 2) & 1, mg = (mr & 63) >> 3;
+    const bool mswap = mj >= 2;
+    const uint32_t m_off = Cfg::M_OFF + ((mr >> 6) * 64 + 2 * (mj & 1) + 32 * (mj >> 1) + 4 * mg + ((n >> 3) & 1)) * 4;
+    const uint32_t m_first = m_off + (mswap ? 16 : 0), m_second = m_off + (mswap ? 0 : 16);
+    const uint32_t msel = mswap ? (mhi ? 0x3276u : 0x1054u) : (mhi ? 0x7632u : 0x5410u);
+    const uint32_t t_lane = tmem_base + ((uint32_t)(quad * 32) << 16);
+
+    const uint32_t aready_leader = mapa_shared(smem_u32(aready_bar), 0);
+    int st = 0, turn = 0;
+    uint32_t phase = 0;
+    for (int item = item0; item < n_items; item += item_step) {
+      const WorkItem w = decode_item<Cfg>(a, prefix, n_seg, n_stripes, item);
+      if (!w.ok) continue;
+      for (int kc = 0; kc < k_chunks; ++kc) {
+        if (turn == team) {
+          mbar_wait(&full_bar[st], phase, dead);
+          const uint32_t sb = smem_base + st * Cfg::STAGE_BYTES;
+          uint32_t e[Cfg::SLABS];
+#pragma unroll
+          for (int s = 0; s < Cfg::SLABS; ++s)
+            e[s] = __byte_perm(lds32(sb + m_first + s * 512), lds32(sb + m_second + s * 512), msel);
+          tc_st4(t_lane + Cfg::META_COL + 4 * st, e[0], e[1], e[2], e[3]);
+          uint32_t sc = 0;
+          if (a.grouped) sc = lds16(sb + s_off) * 0x10001u;
+#pragma unroll
+          for (int s = 0; s < Cfg::SLABS; ++s) {
+            uint32_t q[4], v[8];
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+              const uint32_t w0 = lds32(sb + q_first + s * 1024 + p * 32), w1 = lds32(sb + q_second + s * 1024 + p * 32);
+              q[2 * p] = flip ? w1 : w0;
+              q[2 * p + 1] = flip ? w0 : w1;
+            }
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+              int4x4_to_half2x2(q[m] >> shift, v[m], v[m + 4]);
+              if (a.grouped) {
+                v[m] = hmul2_u32(v[m], sc);
+                v[m + 4] = hmul2_u32(v[m + 4], sc);
+              }
+            }
+            tc_st8(t_lane + Cfg::A_COL + 32 * st + 8 * s, v);
+          }
+          tc_wait_st();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(aready_leader + st * 8);
+        }
+        if (++turn == Cfg::TEAMS) turn = 0;
+        if (++st == STAGES) { st = 0; phase ^= 1; }
+      }
+    }
+  } else if (warp >= Cfg::EPI0) {
+    // ------------------------------ epilogue warps ------------------------------
+    const int ew = warp - Cfg::EPI0;
+    const int quad = warp & 3;
+    const uint32_t accfree_leader = mapa_shared(smem_u32(accfree_bar), 0);
+    uint32_t done[2] = {0, 0};      // tiles published on each accready barrier so far
+    int turn = 0;
     for (int item = item0; item < n_items; item += item_step) {
       WorkItem w = decode_item<Cfg>(a, prefix, n_seg, n_stripes, item);
       w.col0 += my_col;
       if (!w.ok) continue;
+      const int cls = tile_class(w.valid);
+      const int h = cls == 2 ? 0 : turn;
+      if (cls != 2) turn ^= 1;
       for (int t = ew * 32 + lane; t < Cfg::TT; t += Cfg::EPI_WARPS * 32) {
         int r = -1;
         if (t < w.valid) {
@@ -469,8 +461,8 @@ delta_gemm_tcsp_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
       // hardware barrier; the wait spans the whole K loop of the item, so the poller backs off.
       if (ew == 0) {
         uint32_t polls = 0;
-        while (!mbar_try_wait(accready_bar, use & 1)) {
-          __nanosleep(128);
+        while (!mbar_try_wait(&accready_bar[h], done[h] & 1)) {
+          __nanosleep(64);
           if ((polls & 15u) == 0 && *dead) break;
           if (++polls > kMaxPolls) {
             *dead = 1;
@@ -479,29 +471,30 @@ delta_gemm_tcsp_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
           }
         }
       }
+      ++done[h];
       named_bar_sync(4, Cfg::EPI_WARPS * 32);
       tc_fence_after();
-      const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16);
+      const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + h * 128;
       const int nbatch = max(1, (w.valid + 31) >> 5);
-      // The two warps of a quadrant split the 32-token batches; each hands the accumulator back once,
-      // when its last batch is in registers (at once if it has none): the next item's MMAs may then
-      // overwrite it.
-      const int per = (nbatch + 1) >> 1;
-      const int b0 = (ew >> 2) * per, b1 = min(nbatch, b0 + per);
-      auto release = [&]() {
+      // The two warps of a quadrant split the 32-token batches: at the accumulator halves for a 256-token
+      // tile, evenly otherwise.  Each hands a half back once, when its last batch of it is in registers
+      // (at once if it has none): the next item's MMAs may then overwrite it.
+      const int grp = ew >> 2;
+      const int per = cls == 2 ? 4 : (nbatch + 1) >> 1;
+      const int b0 = grp * per, b1 = min(nbatch, b0 + per);
+      auto release = [&](int half) {
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) {
-          if constexpr (PAIR) mbar_arrive_cluster(mapa_shared(smem_u32(accfree_bar), 0));
-          else mbar_arrive(accfree_bar);
-        }
+        if (lane == 0) mbar_arrive_cluster(accfree_leader + half * 8);
       };
-      if (b1 <= b0) release();
+      if (cls == 2) release(grp ^ 1);
+      const int mine = cls == 2 ? grp : h;
+      if (b1 <= b0) release(mine);
       for (int b = b0; b < b1; ++b) {
         uint32_t v[32];
         tc_ld32(taddr + b * 32, v);
         tc_wait_ld();
-        if (b == b1 - 1) release();
+        if (b == b1 - 1) release(mine);
         // Transpose the 32-token x 32-feature block through a private 2 KiB patch of shared memory, so
         // that a lane stores 8 consecutive features (16 bytes) of one token instead of one feature.
         {
@@ -535,19 +528,15 @@ delta_gemm_tcsp_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
         }
       }
       named_bar_sync(4, Cfg::EPI_WARPS * 32);          // rows[] is rewritten for the next item after this
-      ++use;
     }
   }
 
   tc_fence_before();
   __syncthreads();
-  if constexpr (PAIR) cluster_sync_all();   // neither CTA leaves, or frees TMEM, while the other may still touch it
+  cluster_sync_all();   // neither CTA leaves, or frees TMEM, while the other may still touch it
   if (warp == 1) {
     tc_fence_after();
-    if constexpr (PAIR)
-      asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(Cfg::TMEM_COLS) : "memory");
-    else
-      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(Cfg::TMEM_COLS) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(Cfg::TMEM_COLS) : "memory");
   }
 }
 
