@@ -67,7 +67,11 @@ struct TcSpCfg {
   static constexpr int XPOSE_OFF = ROWS_OFF + TT * 4;                     // [EPI_WARPS][32 tokens][32 features] halves
   static constexpr int PREFIX_OFF = XPOSE_OFF + EPI_WARPS * 2048;
   static constexpr int BAR_OFF = PREFIX_OFF + (kMaxSegments + 2) * 4;
-  static constexpr int NUM_BARS = 3 * STAGES + 4;
+  // "Landed" barriers, one per chunk modulo this.  A warp that takes every TEAMS-th chunk can tell the two phases of a
+  // barrier apart only if it has itself passed the barrier's previous use: TMA loads may land out of order, and with
+  // a barrier per stage it could find the phase of a use that another team still waits for.
+  static constexpr int FULL_BARS = STAGES * TEAMS;
+  static constexpr int NUM_BARS = FULL_BARS + 2 * STAGES + 4;
   static constexpr int SMEM_BYTES = BAR_OFF + NUM_BARS * 8 + 16;
   static constexpr int SMEM_ALLOC = SMEM_BYTES + 1024;
   static constexpr uint32_t TMEM_COLS = 512;
@@ -177,8 +181,8 @@ delta_gemm_tcsp_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_c
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   int* rows = reinterpret_cast<int*>(smem + Cfg::ROWS_OFF);
   int* prefix = reinterpret_cast<int*>(smem + Cfg::PREFIX_OFF);
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + Cfg::BAR_OFF);   // TMA data of a stage landed
-  uint64_t* aready_bar = full_bar + STAGES;                                // leader: weights + metadata of a stage in TMEM, both CTAs
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + Cfg::BAR_OFF);   // [FULL_BARS] TMA data of a chunk landed
+  uint64_t* aready_bar = full_bar + Cfg::FULL_BARS;                                // leader: weights + metadata of a stage in TMEM, both CTAs
   uint64_t* empty_bar = aready_bar + STAGES;                               // MMAs of a stage retired
   uint64_t* accready_bar = empty_bar + STAGES;                             // [2] accumulator complete
   uint64_t* accfree_bar = accready_bar + 2;                                // [2] leader: accumulator half drained by both CTAs
@@ -200,8 +204,8 @@ delta_gemm_tcsp_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_c
   }
 
   if (tid == 0) {
+    for (int s = 0; s < Cfg::FULL_BARS; ++s) mbar_init(&full_bar[s], 1);
     for (int s = 0; s < STAGES; ++s) {
-      mbar_init(&full_bar[s], 1);
       mbar_init(&aready_bar[s], 4 * Cfg::CTAS);   // the leader's barrier counts both CTAs' warps of a team
       mbar_init(&empty_bar[s], 1);
     }
@@ -271,7 +275,7 @@ delta_gemm_tcsp_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_c
       prefetch_tmap(&tm_x1);
       prefetch_tmap(&tm_x2);
       const uint64_t pol_x = policy_evict_last();
-      int st = 0;
+      int st = 0, fb = 0;
       uint32_t phase = 0;
       for (int item = item0; item < n_items; item += item_step) {
         const WorkItem w = decode_item<Cfg>(a, prefix, n_seg, n_stripes, item);
@@ -284,9 +288,10 @@ delta_gemm_tcsp_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_c
         for (int kc = 0; kc < k_chunks; ++kc) {
           mbar_wait(&empty_bar[st], phase ^ 1, dead);
           // The stage's one arrival, carrying the bytes of this load and of the weight producer's loads.
-          mbar_arrive_expect_tx(&full_bar[st], stage_tx);
-          tma_load_3d_hint(smem + st * Cfg::STAGE_BYTES + Cfg::B_OFF, tm_x, 0, row0, 2 * kc, &full_bar[st], pol_x);
+          mbar_arrive_expect_tx(&full_bar[fb], stage_tx);
+          tma_load_3d_hint(smem + st * Cfg::STAGE_BYTES + Cfg::B_OFF, tm_x, 0, row0, 2 * kc, &full_bar[fb], pol_x);
           if (++st == STAGES) { st = 0; phase ^= 1; }
+          if (++fb == Cfg::FULL_BARS) fb = 0;
         }
       }
     }
@@ -340,7 +345,7 @@ delta_gemm_tcsp_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_c
       prefetch_tmap(&tm_m);
       if (a.grouped) prefetch_tmap(&tm_s);
       const uint64_t pol_w = policy_evict_first();
-      int st = 0;
+      int st = 0, fb = 0;
       uint32_t phase = 0;
       for (int item = item0; item < n_items; item += item_step) {
         const WorkItem w = decode_item<Cfg>(a, prefix, n_seg, n_stripes, item);
@@ -350,11 +355,12 @@ delta_gemm_tcsp_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_c
           mbar_wait(&empty_bar[st], phase ^ 1, dead);
           uint8_t* sbase = smem + st * Cfg::STAGE_BYTES;
           const int wrow = w.delta * slabs + kc * Cfg::SLABS;
-          tma_load_2d_hint(sbase + Cfg::Q_OFF, &tm_q, (col0 / 64) * 128, wrow, &full_bar[st], pol_w);
-          tma_load_2d_hint(sbase + Cfg::M_OFF, &tm_m, (col0 / 64) * 64, wrow, &full_bar[st], pol_w);
+          tma_load_2d_hint(sbase + Cfg::Q_OFF, &tm_q, (col0 / 64) * 128, wrow, &full_bar[fb], pol_w);
+          tma_load_2d_hint(sbase + Cfg::M_OFF, &tm_m, (col0 / 64) * 64, wrow, &full_bar[fb], pol_w);
           if (a.grouped)
-            tma_load_2d_hint(sbase + Cfg::S_OFF, &tm_s, col0, w.delta * k_chunks + kc, &full_bar[st], pol_w);
+            tma_load_2d_hint(sbase + Cfg::S_OFF, &tm_s, col0, w.delta * k_chunks + kc, &full_bar[fb], pol_w);
           if (++st == STAGES) { st = 0; phase ^= 1; }
+          if (++fb == Cfg::FULL_BARS) fb = 0;
         }
       }
     }
@@ -387,14 +393,14 @@ delta_gemm_tcsp_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_c
     const uint32_t t_lane = tmem_base + ((uint32_t)(quad * 32) << 16);
 
     const uint32_t aready_leader = mapa_shared(smem_u32(aready_bar), 0);
-    int st = 0, turn = 0;
-    uint32_t phase = 0;
+    int st = 0, turn = 0, fb = 0;
+    uint32_t phase = 0;                  // of the "landed" barriers
     for (int item = item0; item < n_items; item += item_step) {
       const WorkItem w = decode_item<Cfg>(a, prefix, n_seg, n_stripes, item);
       if (!w.ok) continue;
       for (int kc = 0; kc < k_chunks; ++kc) {
         if (turn == team) {
-          mbar_wait(&full_bar[st], phase, dead);
+          mbar_wait(&full_bar[fb], phase, dead);
           const uint32_t sb = smem_base + st * Cfg::STAGE_BYTES;
           uint32_t e[Cfg::SLABS];
 #pragma unroll
@@ -428,7 +434,8 @@ delta_gemm_tcsp_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_c
           if (lane == 0) mbar_arrive_cluster(aready_leader + st * 8);
         }
         if (++turn == Cfg::TEAMS) turn = 0;
-        if (++st == STAGES) { st = 0; phase ^= 1; }
+        if (++st == STAGES) st = 0;
+        if (++fb == Cfg::FULL_BARS) { fb = 0; phase ^= 1; }
       }
     }
   } else if (warp >= Cfg::EPI0) {
