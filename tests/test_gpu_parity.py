@@ -833,6 +833,30 @@ def test_base_gemm_with_lora_expand(cuda, M, rank):
     assert _lib().device_status(0) == 0
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("T,K,N,M", [(1, 1024, 264, 0), (100, 1088, 2048, 3), (70, 2048, 5120, 0), (256, 832, 11008, 2),
+                                     (129, 1024, 512, 0), (2300, 128, 768, 0)])
+def test_base_gemm_split_and_order(cuda, T, K, N, M, dtype):
+    """Products with fewer items than CTA pairs, whose K range is shared inside a cluster (four pairs on an item,
+    two on one; uneven ranges; more pairs than token batches), with and
+    without LoRA chunks, writing and adding into y; and one with more token tiles than one group.  Against an fp32
+    torch statement: two roundings to the output type at most, so half of the tolerances of test_base_gemm."""
+    from triteia_b200.ops.matmul._base import base_gemm
+    g = torch.Generator(cuda).manual_seed(T + K + N)
+    x = torch.randn(T, K, device=cuda, generator=g).to(dtype)
+    w = (torch.randn(N, K, device=cuda, generator=g) * 0.05).to(dtype)
+    v = torch.randn(T, 16 * M, device=cuda, generator=g).to(dtype) if M else None
+    b = (torch.randn(16 * M, N, device=cuda, generator=g) * 0.2).to(dtype) if M else None
+    ref = x.float() @ w.float().t() + (v.float() @ b.float() if M else 0)
+    y = base_gemm(x, w, lora_v=v, lora_b=b)
+    tol = ROW_TOL / 2 if dtype == torch.float16 else 1e-2
+    assert oracle.row_rel_err(y.float().cpu().numpy(), ref.cpu().numpy()).max() <= tol
+    assert torch.equal(y, base_gemm(x, w, lora_v=v, lora_b=b))
+    y2 = base_gemm(x, w, lora_v=v, lora_b=b, out=y.clone(), accumulate=True)
+    assert oracle.row_rel_err(y2.float().cpu().numpy(), 2 * ref.cpu().numpy()).max() <= 2 * tol
+    assert _lib().device_status(0) == 0
+
+
 @pytest.mark.parametrize("groupsize", [-1, 128])
 @pytest.mark.parametrize("K,N", [(128, 384), (896, 512)])
 @pytest.mark.parametrize("counts", [(33, 64, 65), (128, 129, 40), (256, 257, 1), (385, 63, 192)])

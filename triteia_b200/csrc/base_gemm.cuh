@@ -59,6 +59,7 @@ struct BaseArgs {
   // operand as it lies in memory).  K is unused, x is the input, the stacked weights come through tm_b.
   const int* seg;
   int n_seg, seg_k;
+  int split_pairs;    // K split: CTA pairs (one cluster) that share an item; 0: a pair takes whole items
 };
 
 // Order of the work items.  CTA pairs take items round-robin, so the items of one round are neighbours:
@@ -101,6 +102,66 @@ __device__ __forceinline__ void tc_mma_f16_pair(uint32_t d_tmem, uint64_t a_desc
       : "memory");
 }
 
+// A 32-token x 32-feature block of results, one feature per lane: convert, transpose through the warp's patch
+// of shared memory, store 16-byte pieces of 8 features.  `old`: the pieces' previous values (accumulate).
+__device__ __forceinline__ void base_store_batch(const BaseArgs& a, __half* patch, const uint32_t (&v)[32], int row0,
+                                                 int valid, int col, int b, int lane, const uint4 (&old)[4]) {
+  if (a.bf16) {
+    __nv_bfloat16* pb = reinterpret_cast<__nv_bfloat16*>(patch);
+#pragma unroll
+    for (int c = 0; c < 32; ++c) pb[c * 32 + lane] = __float2bfloat16_rn(__uint_as_float(v[c]));
+  } else {
+#pragma unroll
+    for (int c = 0; c < 32; ++c) patch[c * 32 + lane] = __float2half_rn(__uint_as_float(v[c]));
+  }
+  __syncwarp();
+  const int f8 = (lane & 3) * 8;                      // feature offset of this lane's 16-byte piece
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int c = i * 8 + (lane >> 2);                // token of the batch
+    const int t = b * 32 + c;
+    if (t < valid && col + f8 < a.N) {
+      uint4 o = *reinterpret_cast<const uint4*>(patch + c * 32 + f8);
+      if (a.accumulate) {
+        if (a.bf16) {
+          __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
+          const __nv_bfloat162* ph = reinterpret_cast<const __nv_bfloat162*>(&old[i]);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float2 p = __bfloat1622float2(oh[e]), q = __bfloat1622float2(ph[e]);
+            oh[e] = __floats2bfloat162_rn(p.x + q.x, p.y + q.y);
+          }
+        } else {
+          __half2* oh = reinterpret_cast<__half2*>(&o);
+          const __half2* ph = reinterpret_cast<const __half2*>(&old[i]);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float2 p = __half22float2(oh[e]), q = __half22float2(ph[e]);
+            oh[e] = __floats2half2_rn(p.x + q.x, p.y + q.y);
+          }
+        }
+      }
+      *reinterpret_cast<uint4*>(a.y + (size_t)(row0 + t) * a.N + col + f8) = o;
+    }
+  }
+  __syncwarp();
+}
+
+__device__ __forceinline__ void st_cluster_v4(uint32_t cluster_addr, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+  asm volatile("st.shared::cluster.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(cluster_addr), "r"(x), "r"(y), "r"(z), "r"(w)
+               : "memory");
+}
+
+// One piece of work of a CTA pair: chunks [kc0, kc1) of an item.
+struct BaseUnit {
+  int item, kc0, kc1;
+};
+
+// SPLIT: for products with fewer items than CTA pairs.  The pairs of a cluster share one item along K; when
+// every accumulator of the cluster is complete, each pair sends the token batches that another pair finishes
+// as fp32 into that pair's shared memory (the stage ring, idle by then) and adds what it receives for its own
+// batches in the order of the ranges.  Everything stays inside the cluster: no workspace, no counters.
+template <bool SPLIT>
 __global__ void __launch_bounds__(BaseCfg::THREADS, 1)
 base_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w,
                  const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_b,
@@ -166,11 +227,12 @@ base_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
   }
   tc_fence_before();
   __syncthreads();
-  cluster_sync_all();     // both CTAs' barriers exist before any remote arrive
+  cluster_sync_all();     // the cluster's barriers exist before any remote arrive
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  const uint32_t rank = cluster_ctarank();
+  const uint32_t crank = cluster_ctarank();
+  const uint32_t rank = crank & 1, leader = crank & ~1u;   // place in the pair, the pair's leader CTA
   const int n_stripes = (a.N + 255) / 256;            // an item: 256 features (128 per CTA) x one token tile
   const int n_tiles = a.seg != nullptr ? prefix[n_seg] : (a.T + a.tt - 1) / a.tt;
   const int n_items = n_tiles * n_stripes;
@@ -198,6 +260,17 @@ base_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
   const int kl = ((a.seg != nullptr ? a.seg_k : a.kv) + Cfg::KC - 1) / Cfg::KC;         // MN-major chunks (LoRA)
   const int k_chunks = kw + kl;
   const uint32_t smem_base = smem_u32(smem);
+  // The u-th unit of work of this CTA's pair.
+  const int part = (int)(crank >> 1), parts = SPLIT ? a.split_pairs : 1;
+  auto unit = [&](int u, BaseUnit& w) -> bool {
+    if constexpr (SPLIT) {
+      w = BaseUnit{(int)blockIdx.x / (2 * parts), part * k_chunks / parts, (part + 1) * k_chunks / parts};
+      return u == 0 && w.item < n_items;
+    } else {
+      w = BaseUnit{item0 + u * item_step, 0, k_chunks};
+      return w.item < n_items;
+    }
+  };
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
@@ -214,16 +287,17 @@ base_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
       const uint32_t stage_tx = Cfg::A_BYTES + half_tt * Cfg::KC * 2;
       int st = 0;
       uint32_t phase = 0;
-      for (int item = item0; item < n_items; item += item_step) {
+      BaseUnit w;
+      for (int u = 0; unit(u, w); ++u) {
         int tile, stripe;
-        base_item(item, n_tiles, n_stripes, a.group, tile, stripe);
+        base_item(w.item, n_tiles, n_stripes, a.group, tile, stripe);
         int row0, valid, sg;
         tile_rows(tile, row0, valid, sg);
         row0 += (int)rank * half_tt;
         const int col0 = stripe * 256 + (int)rank * 128;
         const int wrow0 = a.seg != nullptr ? sg * a.seg_k : 0;      // first row of this segment's weight
         const CUtensorMap* tm_in = a.seg != nullptr ? &tm_x : &tm_v;
-        for (int kc = 0; kc < k_chunks; ++kc) {
+        for (int kc = w.kc0; kc < w.kc1; ++kc) {
           mbar_wait(&empty_bar[st], phase ^ 1, dead);
           uint8_t* sbase = smem + st * Cfg::STAGE_BYTES;
           mbar_arrive_expect_tx(&full_bar[st], stage_tx);
@@ -252,12 +326,13 @@ base_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
       uint32_t phase = 0;
       uint32_t use[2] = {0, 0};
       int local = 0;
-      for (int item = item0; item < n_items; item += item_step) {
+      BaseUnit w;
+      for (int u = 0; unit(u, w); ++u) {
         const int buf = local & 1;
         mbar_wait_cluster(&accfree_bar[buf], (use[buf] & 1) ^ 1, dead);
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + buf * Cfg::MAX_TT;
-        for (int kc = 0; kc < k_chunks; ++kc) {
+        for (int kc = w.kc0; kc < w.kc1; ++kc) {
           mbar_wait_cluster(&ready_bar[st], phase, dead);
           tc_fence_after();
           const uint32_t sb = smem_base + st * Cfg::STAGE_BYTES;
@@ -266,19 +341,19 @@ base_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
             const uint64_t adesc = tc_smem_desc(sb + Cfg::A_OFF);
 #pragma unroll
             for (int k = 0; k < Cfg::KC / 16; ++k)   // +32 bytes of K per instruction = +2 in the address field
-              tc_mma_f16_pair(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (kc > 0 || k > 0) ? 1u : 0u);
+              tc_mma_f16_pair(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (kc > w.kc0 || k > 0) ? 1u : 0u);
           } else {
 #pragma unroll
             for (int k = 0; k < Cfg::KC / 16; ++k) {  // 16 K rows of 128 bytes per instruction
               // 64-feature halves 8 KiB apart, 8-row K groups 1 KiB apart
               const uint64_t adesc = tc_smem_desc_mn(sb + Cfg::A_OFF + k * 2048, 8192, 1024);
-              tc_mma_f16_pair(d_tmem, adesc, bdesc + 2 * k, idesc_mn, (kc > 0 || k > 0) ? 1u : 0u);
+              tc_mma_f16_pair(d_tmem, adesc, bdesc + 2 * k, idesc_mn, (kc > w.kc0 || k > 0) ? 1u : 0u);
             }
           }
-          tc_commit_pair(&empty_bar[st]);
+          tc_commit_pair(&empty_bar[st], (uint16_t)(3u << leader));
           if (++st == STAGES) { st = 0; phase ^= 1; }
         }
-        tc_commit_pair(&accready_bar[buf]);
+        tc_commit_pair(&accready_bar[buf], (uint16_t)(3u << leader));
         ++use[buf];
         ++local;
       }
@@ -286,11 +361,12 @@ base_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
   } else if (warp == 2 + Cfg::EPI_WARPS) {
     // ------------------------------ stage relay: this CTA's data landed -> the leader ------------------------------
     if (lane == 0) {
-      const uint32_t ready_leader = mapa_shared(smem_u32(ready_bar), 0);
+      const uint32_t ready_leader = mapa_shared(smem_u32(ready_bar), leader);
       int st = 0;
       uint32_t phase = 0;
-      for (int item = item0; item < n_items; item += item_step) {
-        for (int kc = 0; kc < k_chunks; ++kc) {
+      BaseUnit w;
+      for (int u = 0; unit(u, w); ++u) {
+        for (int kc = w.kc0; kc < w.kc1; ++kc) {
           mbar_wait(&full_bar[st], phase, dead);
           mbar_arrive_cluster(ready_leader + st * 8);
           if (++st == STAGES) { st = 0; phase ^= 1; }
@@ -301,12 +377,18 @@ base_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
     // ------------------------------ epilogue warps ------------------------------
     const int ew = warp - 2;
     const int quad = warp & 3;                        // TMEM lanes this warp may touch: 32 * quad .. + 31
-    const uint32_t accfree_leader = mapa_shared(smem_u32(accfree_bar), 0);
+    const uint32_t accfree_leader = mapa_shared(smem_u32(accfree_bar), leader);
+    __half* patch = reinterpret_cast<__half*>(smem + Cfg::XPOSE_OFF + ew * 2048);
     uint32_t use[2] = {0, 0};
     int local = 0;
-    for (int item = item0; item < n_items; item += item_step) {
+    if constexpr (SPLIT) {
+      if (ew == 0) mbar_wait(&accready_bar[0], 0, dead);
+      named_bar_sync(4, Cfg::EPI_WARPS * 32);
+    }
+    BaseUnit w;
+    for (int u = 0; !SPLIT && unit(u, w); ++u) {
       int tile, stripe;
-        base_item(item, n_tiles, n_stripes, a.group, tile, stripe);
+      base_item(w.item, n_tiles, n_stripes, a.group, tile, stripe);
       int row0, valid, sg;
       tile_rows(tile, row0, valid, sg);
       const int col0 = stripe * 256 + (int)rank * 128;
@@ -365,54 +447,89 @@ base_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
           if (lane == 0) mbar_arrive_cluster(accfree_leader + buf * 8);
         }
         if (b >= b1) continue;
-        __half* patch = reinterpret_cast<__half*>(smem + Cfg::XPOSE_OFF + ew * 2048);
-        if (a.bf16) {
-          __nv_bfloat16* pb = reinterpret_cast<__nv_bfloat16*>(patch);
-#pragma unroll
-          for (int c = 0; c < 32; ++c) pb[c * 32 + lane] = __float2bfloat16_rn(__uint_as_float(v[c]));
-        } else {
-#pragma unroll
-          for (int c = 0; c < 32; ++c) patch[c * 32 + lane] = __float2half_rn(__uint_as_float(v[c]));
-        }
-        __syncwarp();
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int c = i * 8 + (lane >> 2);          // token of the batch
-          uint4* yp = piece(b, i);
-          if (yp != nullptr) {
-            uint4 o = *reinterpret_cast<const uint4*>(patch + c * 32 + f8);
-            if (a.accumulate) {
-              if (a.bf16) {
-                __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
-                const __nv_bfloat162* ph = reinterpret_cast<const __nv_bfloat162*>(&old[k][i]);
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  const float2 p = __bfloat1622float2(oh[e]), q = __bfloat1622float2(ph[e]);
-                  oh[e] = __floats2bfloat162_rn(p.x + q.x, p.y + q.y);
-                }
-              } else {
-                __half2* oh = reinterpret_cast<__half2*>(&o);
-                const __half2* ph = reinterpret_cast<const __half2*>(&old[k][i]);
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  const float2 p = __half22float2(oh[e]), q = __half22float2(ph[e]);
-                  oh[e] = __floats2half2_rn(p.x + q.x, p.y + q.y);
-                }
-              }
-            }
-            *yp = o;
-          }
-        }
-        __syncwarp();
+        base_store_batch(a, patch, v, row0, valid, col0 + quad * 32, b, lane, old[k]);
       }
       ++use[buf];
       ++local;
     }
   }
 
+  if constexpr (SPLIT) {
+    cluster_sync_all();     // every accumulator of the cluster is complete: the stage rings are free
+    const bool epi = warp >= 2 && warp < 2 + Cfg::EPI_WARPS;
+    const int ew = warp - 2, quad = warp & 3, grp = ew >> 2;
+    BaseUnit w;
+    unit(0, w);
+    int tile, stripe, row0, valid, sg;
+    base_item(w.item, n_tiles, n_stripes, a.group, tile, stripe);
+    tile_rows(tile, row0, valid, sg);
+    const int col0 = stripe * 256 + (int)rank * 128 + quad * 32;
+    const int nbatch = (valid + 31) >> 5;
+    const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16);
+    // Part p finishes batches [p * nbatch / parts, (p + 1) * nbatch / parts).  A received block: sending part
+    // (without one's own), batch inside the slice, lane quadrant, 4 KiB each; 96 KiB at most.
+    const uint32_t slice_max = (uint32_t)((nbatch + parts - 1) / parts);
+    auto block_at = [&](int sender, int receiver, int in_slice) {
+      const uint32_t from = (uint32_t)(sender < receiver ? sender : sender - 1);
+      return ((from * slice_max + in_slice) * 4 + quad) * 4096 + lane * 16;
+    };
+    if (epi) {
+      tc_fence_after();
+      for (int p = 0; p < parts; ++p) {
+        if (p == part) continue;
+        const uint32_t dst = mapa_shared(smem_base, (uint32_t)(2 * p) + rank);
+        const int lo = p * nbatch / parts, hi = (p + 1) * nbatch / parts;
+        for (int b = lo + grp; b < hi; b += 2) {
+          uint32_t v[32];
+          tc_ld32(taddr + b * 32, v);
+          tc_wait_ld();
+          const uint32_t at = dst + block_at(part, p, b - lo);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) st_cluster_v4(at + i * 512, v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        }
+      }
+    }
+    cluster_sync_all();     // every partial sum has arrived
+    if (epi) {
+      __half* patch = reinterpret_cast<__half*>(smem + Cfg::XPOSE_OFF + ew * 2048);
+      const int lo = part * nbatch / parts, hi = (part + 1) * nbatch / parts;
+      for (int b = lo + grp; b < hi; b += 2) {
+        uint4 old[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int t = b * 32 + i * 8 + (lane >> 2), col = col0 + (lane & 3) * 8;
+          old[i] = make_uint4(0, 0, 0, 0);
+          if (a.accumulate && t < valid && col < a.N) old[i] = *reinterpret_cast<const uint4*>(a.y + (size_t)(row0 + t) * a.N + col);
+        }
+        uint32_t own[32], v[32];
+        tc_ld32(taddr + b * 32, own);
+        tc_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] = 0u;
+        for (int p = 0; p < parts; ++p) {
+          if (p == part) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) + __uint_as_float(own[i]));
+          } else {
+            const uint32_t at = smem_base + block_at(p, part, b - lo);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const uint4 r = lds128(at + i * 512);
+              v[4 * i] = __float_as_uint(__uint_as_float(v[4 * i]) + __uint_as_float(r.x));
+              v[4 * i + 1] = __float_as_uint(__uint_as_float(v[4 * i + 1]) + __uint_as_float(r.y));
+              v[4 * i + 2] = __float_as_uint(__uint_as_float(v[4 * i + 2]) + __uint_as_float(r.z));
+              v[4 * i + 3] = __float_as_uint(__uint_as_float(v[4 * i + 3]) + __uint_as_float(r.w));
+            }
+          }
+        }
+        base_store_batch(a, patch, v, row0, valid, col0, b, lane, old);
+      }
+    }
+  }
+
   tc_fence_before();
   __syncthreads();
-  cluster_sync_all();   // neither CTA leaves, or frees TMEM, while the other may still touch it
+  cluster_sync_all();   // no CTA leaves, or frees TMEM, while another may still touch it
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(Cfg::TMEM_COLS) : "memory");
@@ -485,13 +602,59 @@ __global__ void __launch_bounds__(kShrinkThreads) lora_shrink_rows_kernel(__half
 
 static_assert(BaseCfg::SMEM_ALLOC <= 232448, "shared memory budget of one sm_100 CTA");
 
-static int base_gemm_launch_args(const BaseArgs& a, const CUtensorMap& tx, const CUtensorMap& tw, const CUtensorMap& tv,
+// Clusters of 2 * pairs CTAs that the device holds at once (asked once per device and cluster size).
+static int max_split_clusters(int dev, int pairs) {
+  static std::atomic<int> cached[64][8];
+  if (dev < 0 || dev >= 64 || pairs < 1 || pairs >= 8) return 0;
+  int v = cached[dev][pairs].load(std::memory_order_relaxed);
+  if (v == 0) {
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(2 * pairs);
+    lc.blockDim = dim3(BaseCfg::THREADS);
+    lc.dynamicSmemBytes = BaseCfg::SMEM_ALLOC;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2 * pairs;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, base_gemm_kernel<true>, &lc) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    v = n + 1;
+    cached[dev][pairs].store(v, std::memory_order_relaxed);
+  }
+  return v - 1;
+}
+
+// CTA pairs that share an item of a product with `items` items of `k_chunks` chunks: four or two, when all clusters
+// run in one round and a pair keeps at least four chunks; otherwise 0.  The exchange costs about 4 us, a chunk 0.27.
+// Measured (CUDA events, cold L2; whole items -> split): 100 x 2048 x 2048 20.5 -> 18.4 us, 16 x 4096 x 4096
+// 28.7 -> 24.6, 64 x 4096 x 5120 29.5 -> 25.3, 1 x 11008 x 4096 60.4 -> 39.8.  Three pairs on two items, which
+// would use the pairs that 43 items leave idle, lost: 256 x 4096 x 11008 34.8 -> 38.9, 256 x 2048 x 9216 23.4 -> 31.5.
+static int choose_split(int dev, long long items, int k_chunks) {
+  for (int p = 4; p >= 2; p -= 2)
+    if (k_chunks >= 4 * p && items <= max_split_clusters(dev, p)) return p;
+  return 0;
+}
+
+static int base_gemm_launch_args(BaseArgs a, const CUtensorMap& tx, const CUtensorMap& tw, const CUtensorMap& tv,
                                  const CUtensorMap& tb, long long items, int dev, cudaStream_t stream) {
-  static std::atomic<bool> attr_set[64];
-  if (!ensure_smem_attr(base_gemm_kernel, dev, BaseCfg::SMEM_ALLOC, attr_set)) return TRB_ERR_CUDA;
+  static std::atomic<bool> attr_set[64], attr_set_split[64];
+  if (!ensure_smem_attr(base_gemm_kernel<false>, dev, BaseCfg::SMEM_ALLOC, attr_set)) return TRB_ERR_CUDA;
+  if (!ensure_smem_attr(base_gemm_kernel<true>, dev, BaseCfg::SMEM_ALLOC, attr_set_split)) return TRB_ERR_CUDA;
   int pairs = sm_count(dev) / 2;
   if (pairs < 1) pairs = 1;
   if (items < pairs) pairs = (int)(items > 0 ? items : 1);
+  int cluster = 2;
+  if (a.seg == nullptr) a.split_pairs = choose_split(dev, items, a.K / BaseCfg::KC + (a.kv + BaseCfg::KC - 1) / BaseCfg::KC);
+  if (a.split_pairs > 0) {
+    cluster = 2 * a.split_pairs;
+    pairs = a.split_pairs * (int)items;
+  }
   cudaLaunchConfig_t lc = {};
   lc.gridDim = dim3(2 * pairs);
   lc.blockDim = dim3(BaseCfg::THREADS);
@@ -501,12 +664,15 @@ static int base_gemm_launch_args(const BaseArgs& a, const CUtensorMap& tx, const
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // the kernel waits (pdl_wait) before it reads
   at[0].val.programmaticStreamSerializationAllowed = 1;
   at[1].id = cudaLaunchAttributeClusterDimension;
-  at[1].val.clusterDim.x = 2;
+  at[1].val.clusterDim.x = cluster;
   at[1].val.clusterDim.y = 1;
   at[1].val.clusterDim.z = 1;
   lc.attrs = at;
   lc.numAttrs = 2;
-  return cudaLaunchKernelEx(&lc, base_gemm_kernel, tx, tw, tv, tb, a) == cudaSuccess ? TRB_OK : TRB_ERR_CUDA;
+  return cudaLaunchKernelEx(&lc, a.split_pairs > 0 ? base_gemm_kernel<true> : base_gemm_kernel<false>, tx, tw, tv, tb, a) ==
+                 cudaSuccess
+             ? TRB_OK
+             : TRB_ERR_CUDA;
 }
 
 static int token_tile_for(int rows) { return rows <= 32 ? 32 : rows <= 64 ? 64 : rows <= 128 ? 128 : 256; }

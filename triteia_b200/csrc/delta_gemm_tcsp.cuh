@@ -164,9 +164,10 @@ __device__ __forceinline__ void tc_mma_sp_f16_pair(uint32_t d_tmem, uint32_t a_t
       : "memory");
 }
 // Arrive on the barrier at this shared-memory offset in both CTAs once the pair's MMAs issued so far retire.
-__device__ __forceinline__ void tc_commit_pair(uint64_t* bar) {
+// (`mask`: the pair's CTAs by their rank in the cluster).
+__device__ __forceinline__ void tc_commit_pair(uint64_t* bar, uint16_t mask = 3) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-               ::"r"(smem_u32(bar)), "h"((uint16_t)3)
+               ::"r"(smem_u32(bar)), "h"(mask)
                : "memory");
 }
 
