@@ -97,8 +97,8 @@ __device__ __forceinline__ void tc_mma_f16_pair(uint32_t d_tmem, uint64_t a_desc
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 
@@ -317,7 +317,8 @@ base_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer (leader CTA) ------------------------------
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
+      const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
       // D fp32, A and B fp16 / bf16; N = token tile, M = 256; bit 15: A is MN-major (the LoRA chunks)
       const uint32_t fmt = a.bf16 ? 1u : 0u;           // operand format field: 0 = fp16, 1 = bf16
       const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | (((uint32_t)a.tt >> 3) << 17) | ((256u >> 4) << 24);
@@ -331,29 +332,33 @@ base_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
         const int buf = local & 1;
         mbar_wait_cluster(&accfree_bar[buf], (use[buf] & 1) ^ 1, dead);
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + buf * Cfg::MAX_TT;
+        const uint32_t d_tmem = tmem + buf * Cfg::MAX_TT;
         for (int kc = w.kc0; kc < w.kc1; ++kc) {
           mbar_wait_cluster(&ready_bar[st], phase, dead);
           tc_fence_after();
           const uint32_t sb = smem_base + st * Cfg::STAGE_BYTES;
           const uint64_t bdesc = tc_smem_desc(sb + Cfg::B_OFF);
-          if (kc < kw) {
-            const uint64_t adesc = tc_smem_desc(sb + Cfg::A_OFF);
+          if (elect_one()) {
+            if (kc < kw) {
+              const uint64_t adesc = tc_smem_desc(sb + Cfg::A_OFF);
 #pragma unroll
-            for (int k = 0; k < Cfg::KC / 16; ++k)   // +32 bytes of K per instruction = +2 in the address field
-              tc_mma_f16_pair(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (kc > w.kc0 || k > 0) ? 1u : 0u);
-          } else {
+              for (int k = 0; k < Cfg::KC / 16; ++k)   // +32 bytes of K per instruction = +2 in the address field
+                tc_mma_f16_pair(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (kc > w.kc0 || k > 0) ? 1u : 0u);
+            } else {
 #pragma unroll
-            for (int k = 0; k < Cfg::KC / 16; ++k) {  // 16 K rows of 128 bytes per instruction
-              // 64-feature halves 8 KiB apart, 8-row K groups 1 KiB apart
-              const uint64_t adesc = tc_smem_desc_mn(sb + Cfg::A_OFF + k * 2048, 8192, 1024);
-              tc_mma_f16_pair(d_tmem, adesc, bdesc + 2 * k, idesc_mn, (kc > w.kc0 || k > 0) ? 1u : 0u);
+              for (int k = 0; k < Cfg::KC / 16; ++k) {  // 16 K rows of 128 bytes per instruction
+                // 64-feature halves 8 KiB apart, 8-row K groups 1 KiB apart
+                const uint64_t adesc = tc_smem_desc_mn(sb + Cfg::A_OFF + k * 2048, 8192, 1024);
+                tc_mma_f16_pair(d_tmem, adesc, bdesc + 2 * k, idesc_mn, (kc > w.kc0 || k > 0) ? 1u : 0u);
+              }
             }
+            tc_commit_pair(&empty_bar[st], (uint16_t)(3u << leader));
           }
-          tc_commit_pair(&empty_bar[st], (uint16_t)(3u << leader));
+          __syncwarp();
           if (++st == STAGES) { st = 0; phase ^= 1; }
         }
-        tc_commit_pair(&accready_bar[buf], (uint16_t)(3u << leader));
+        if (elect_one()) tc_commit_pair(&accready_bar[buf], (uint16_t)(3u << leader));
+        __syncwarp();
         ++use[buf];
         ++local;
       }

@@ -159,8 +159,8 @@ __device__ __forceinline__ void tc_mma_sp_f16_pair(uint32_t d_tmem, uint32_t a_t
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.sp.cta_group::2.kind::f16 [%0], [%1], %2, [%6], %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u), "r"(e_tmem)
+      "tcgen05.mma.sp.cta_group::2.kind::f16 [%0], [%1], %2, [%5], %3, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(e_tmem)
       : "memory");
 }
 // Arrive on the barrier at this shared-memory offset in both CTAs once the pair's MMAs issued so far retire.
@@ -298,14 +298,15 @@ delta_gemm_tcsp_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_c
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
+      const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
       int st = 0;
       uint32_t phase = 0, used[2] = {0, 0};
       int turn = 0;
       for (int item = item0; item < n_items; item += item_step) {
         const WorkItem w = decode_item<Cfg>(a, prefix, n_seg, n_stripes, item);
         if (!w.ok) continue;
-        const int cls = tile_class(w.valid);
+        const int cls = __shfl_sync(0xffffffffu, tile_class(w.valid), 0);
         // A 256-token tile takes both halves of the accumulator columns, smaller ones take turns.
         const int h = cls == 2 ? 0 : turn;
         mbar_wait_cluster(&accfree_bar[h], (used[h] & 1) ^ 1, dead);
@@ -317,7 +318,7 @@ delta_gemm_tcsp_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_c
           turn ^= 1;
         }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + h * 128;
+        const uint32_t d_tmem = tmem + h * 128;
         const uint32_t idesc = (1u << 4) | ((uint32_t)(8 << cls) << 17) | ((256u >> 4) << 24) | (1u << 2);   // N = 64 << cls
         const uint32_t khalf = (32u << cls) * 128u >> 4;      // descriptor step to the second 64-K half
         for (int kc = 0; kc < k_chunks; ++kc) {
@@ -326,16 +327,20 @@ delta_gemm_tcsp_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_c
           mbar_wait_cluster(&aready_bar[st], phase, dead);
           tc_fence_after();
           const uint64_t bdesc = tc_smem_desc(smem_base + st * Cfg::STAGE_BYTES + Cfg::B_OFF);
-          const uint32_t a_tmem = tmem_base + Cfg::A_COL + 32 * st;
-          const uint32_t e_tmem = tmem_base + Cfg::META_COL + 4 * st;
+          const uint32_t a_tmem = tmem + Cfg::A_COL + 32 * st;
+          const uint32_t e_tmem = tmem + Cfg::META_COL + 4 * st;
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < Cfg::SLABS; ++k)   // per instruction: 8 columns of weights, 64 bytes of B, one metadata column
-            tc_mma_sp_f16_pair(d_tmem, a_tmem + 8 * k, bdesc + (k >> 1) * khalf + 4 * (k & 1), e_tmem + (k & 2),
-                               idesc | (k & 1), (kc > 0 || k > 0) ? 1u : 0u);
-          tc_commit_pair(&empty_bar[st]);
+            for (int k = 0; k < Cfg::SLABS; ++k)   // per instruction: 8 columns of weights, 64 bytes of B, one metadata column
+              tc_mma_sp_f16_pair(d_tmem, a_tmem + 8 * k, bdesc + (k >> 1) * khalf + 4 * (k & 1), e_tmem + (k & 2),
+                                 idesc | (k & 1), (kc > 0 || k > 0) ? 1u : 0u);
+            tc_commit_pair(&empty_bar[st]);
+          }
+          __syncwarp();
           if (++st == STAGES) { st = 0; phase ^= 1; }
         }
-        tc_commit_pair(&accready_bar[h]);
+        if (elect_one()) tc_commit_pair(&accready_bar[h]);
+        __syncwarp();
       }
     }
   } else if (warp == 2) {
