@@ -301,6 +301,12 @@ int trb_base_gemm(const void* x, const void* base_weight, void* y, int num_token
 int trb_sgmv_stacked(void* y, const void* x, const void* w, const void* s, int num_problems, int num_rows,
                      int d_in, int d_out, int max_rows, int accumulate, int dtype, int dev, void* stream);
 
+/* Segment offsets of adapter ids for the segmented LoRA products: s[i] = number of ids in [-1, i) for i = 0 ..
+ * num_adapters (int32 [num_adapters + 1]; ids outside [-1, num_adapters) are not counted).  The device form of the
+ * host loop of triteia/python/ops/matmul/lora.py:63-78.  num_adapters <= 8191. */
+int trb_segments(const void* indices, int index_is_64bit, int num_tokens, int num_adapters, void* s, int dev,
+                 void* stream);
+
 /* Shrink half of the indexed LoRA, written as the operand of trb_base_gemm: row b of v[B, v_cols]
  * (fp16) becomes zero except columns [id * rank, (id + 1) * rank) = scale * x[b] @ A[id], with
  * A [M, h1, rank] fp16 and id = indices[b] (int32, or int64 when index_is_64bit); ids outside

@@ -1008,3 +1008,12 @@ def test_sgmv_stacked_ragged_segments(cuda, rank, dtype):
     assert err.max() <= (ROW_TOL if dtype == torch.float16 else 3e-2), f"row rel err {err.max():.4g}"
     assert torch.equal(y[:lead], y0[:lead])
     assert _lib().device_status(0) == 0
+
+
+@pytest.mark.parametrize("T,M", [(0, 3), (1, 1), (33, 5), (1025, 16), (8192, 1000)])
+def test_segment_offsets(cuda, T, M):
+    """Offsets of grouped ids against the counting statement in torch, ids outside [-1, M) included: whole numbers."""
+    from triteia_b200.ops.matmul.lora import segment_offsets
+    for dtype in (torch.int32, torch.int64):
+        ids = torch.from_numpy(np.sort(np.random.default_rng(T).integers(-3, M + 2, T))).to(dtype)
+        assert torch.equal(segment_offsets(ids.to(cuda), M).cpu(), segment_offsets(ids, M))

@@ -706,12 +706,23 @@ static int base_gemm_launch(const void* x, const void* w, void* y, int T, int N,
   return base_gemm_launch_args(a, tx, tw, tv, tb, items, dev, stream);
 }
 
+// Token tile of the segmented form: the smallest whose items still run in one round (a round of narrow tiles streams
+// the input over all SMs: LoRA shrink, one stripe), otherwise the widest that the longest segment fills.
+// lora_sgmv of 7001 tokens, 16 adapters of rank 64, together with the offsets in one kernel: 1.18x -> 1.26x of
+// the call as it was without either (985 us).
+static int segment_tile_for(int rows, int T, int n_seg, int n_stripes, int dev) {
+  const int widest = token_tile_for(rows);
+  for (int tt = 32; tt < widest; tt *= 2)
+    if (((long long)T / tt + n_seg) * n_stripes <= sm_count(dev) / 2) return tt;
+  return widest;
+}
+
 // Segmented form: y[seg[i] : seg[i + 1]] (+)= x[same rows] @ w[i], w stacked [n_seg, d_in, d_out].
 static int sgmv_stacked_launch(void* y, const void* x, const void* w, const int* seg, int n_seg, int T, int d_in,
                                int d_out, int max_rows, int accumulate, int bf16, int dev, cudaStream_t stream) {
   BaseArgs a{};
   a.T = T; a.N = d_out; a.K = 0; a.kv = 0;
-  a.tt = token_tile_for(max_rows > 0 ? max_rows : T);
+  a.tt = segment_tile_for(max_rows > 0 ? max_rows : T, T, n_seg, (d_out + 255) / 256, dev);
   a.group = kTileGroup;
   a.y = (__half*)y;
   a.accumulate = accumulate;

@@ -224,6 +224,33 @@ route_kernel(const RouteSrc src, int T, int D, int W, int TT, int* __restrict__ 
   }
 }
 
+// Segment offsets of adapter ids: s[i] = number of ids in [-1, i), i = 0 .. M (ids outside [-1, M) count nowhere),
+// which are the row ranges when the ids are grouped in increasing order.  One CTA: a histogram in shared memory,
+// equal neighbours added once per warp step, and a scan.  Bound by its chain of a few dependent loads (T / 1024 per
+// thread); the torch statement it stands for compares T x (M + 1) pairs and reduces them, 40 us and three launches
+// at 7001 ids and 16 adapters.
+template <class IdxT>
+__global__ void __launch_bounds__(kRouteThreads, 1)
+segments_kernel(const IdxT* __restrict__ ids, int T, int M, int* __restrict__ s) {
+  extern __shared__ int sm[];            // [M + 2] counts of -1, 0, .., M - 1, and a zero
+  __shared__ int warp_tot[33];
+  const int tid = threadIdx.x, lane = tid & 31;
+  pdl_launch_dependents();
+  for (int i = tid; i < M + 2; i += blockDim.x) sm[i] = 0;
+  __syncthreads();
+  pdl_wait();
+  for (int base = 0; base < T; base += blockDim.x) {
+    const int t = base + tid;
+    const long long id = t < T ? (long long)ids[t] : -2;
+    const int bin = id >= -1 && id < M ? (int)id + 1 : -1;
+    const unsigned same = __match_any_sync(0xffffffffu, bin);
+    if (bin >= 0 && (same & ((1u << lane) - 1)) == 0) atomicAdd(&sm[bin], __popc(same));
+  }
+  __syncthreads();
+  block_exclusive_scan(sm, M + 2, warp_tot);
+  for (int i = tid; i <= M; i += blockDim.x) s[i] = sm[i + 1];
+}
+
 // x_sorted[p] = x[perm[p]] for every sorted position; optionally zero y rows whose id is -1.
 __global__ void gather_rows_kernel(const uint4* __restrict__ x, const int* __restrict__ perm,
                                    const int* __restrict__ counters, uint4* __restrict__ x_sorted,
@@ -257,6 +284,28 @@ extern "C" int trb_route_max_tiles(int num_tokens, int num_deltas, int tile_toke
   if (num_tokens <= 0 || tile_tokens <= 0) return 0;
   const int segs = num_tokens < num_deltas ? num_tokens : num_deltas;
   return num_tokens / tile_tokens + segs;
+}
+
+extern "C" int trb_segments(const void* indices, int index_is_64bit, int num_tokens, int num_adapters, void* s, int dev,
+                            void* stream_v) {
+  using namespace trb;
+  if (num_tokens < 0 || num_adapters < 0 || !s || (num_tokens > 0 && !indices)) return TRB_ERR_BAD_ARG;
+  if (num_adapters > 8191) return TRB_ERR_KERN_SHAPE;
+  if (cudaSetDevice(dev) != cudaSuccess) return TRB_ERR_CUDA;
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(1);
+  lc.blockDim = dim3(kRouteThreads);
+  lc.dynamicSmemBytes = (size_t)(num_adapters + 2) * sizeof(int);
+  lc.stream = (cudaStream_t)stream_v;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // the kernel waits (pdl_wait) before it reads or writes
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = at;
+  lc.numAttrs = 1;
+  const cudaError_t e = index_is_64bit
+                            ? cudaLaunchKernelEx(&lc, segments_kernel<int64_t>, (const int64_t*)indices, num_tokens, num_adapters, (int*)s)
+                            : cudaLaunchKernelEx(&lc, segments_kernel<int32_t>, (const int32_t*)indices, num_tokens, num_adapters, (int*)s);
+  return e == cudaSuccess ? TRB_OK : TRB_ERR_CUDA;
 }
 
 namespace trb {

@@ -48,6 +48,19 @@ def lora_bgmv(weights_A, weights_B, x, indices, base_weight=None, layer_idx=0, s
     return lora_indexed(y, x, weights_A, weights_B, indices, scale)
 
 
+def segment_offsets(indices, M):
+    """int32 [M + 1]: s[i] = number of ids in [-1, i), the first row of adapter i when the ids are grouped."""
+    if indices.is_cuda and indices.dtype in (torch.int32, torch.int64) and indices.dim() == 1 and M <= 8191:
+        indices = indices.contiguous()
+        s = torch.empty(M + 1, dtype=torch.int32, device=indices.device)
+        _lib.check(lib.trb_segments(ptr(indices), int(indices.dtype == torch.int64), indices.numel(), M, ptr(s),
+                                    dev_of(indices), stream_of(indices)), "segments")
+        return s
+    ids = torch.arange(-1, M, device=indices.device, dtype=indices.dtype)
+    counts = (indices[:, None] == ids[None, :]).sum(0)           # [-1, 0, .., M-1]
+    return torch.cumsum(counts, 0).to(torch.int32)
+
+
 def sgmv_stacked(y, x, weights, seg, accumulate=True, max_rows=0):
     """In place: y[seg[i]:seg[i+1]] (+)= x[seg[i]:seg[i+1]] @ weights[i]; weights [S, d_in, d_out]
     contiguous, seg int32 [S + 1] on the device."""
@@ -68,9 +81,7 @@ def lora_sgmv(weights_A, weights_B, x, indices, base_weight=None, layer_idx=0):
     `add_lora_sgmv_cutlass`, triteia/python/capi/punica.py:4-32, which stays available in capi)."""
     y = _base(x, base_weight, weights_B.shape[2])
     M, _, rank = weights_A.shape
-    ids = torch.arange(-1, M, device=x.device, dtype=indices.dtype)
-    counts = (indices[:, None] == ids[None, :]).sum(0)           # [-1, 0, .., M-1]
-    s = torch.cumsum(counts, 0).to(torch.int32)                   # s[i] = first row of adapter i
+    s = segment_offsets(indices, M)
     if not (weights_A.is_contiguous() and weights_B.is_contiguous() and x.is_contiguous()):
         weights_A, weights_B, x = weights_A.contiguous(), weights_B.contiguous(), x.contiguous()
     if rank % 8 != 0 or x.shape[1] % 8 != 0 or y.shape[1] % 8 != 0 or M > 1024:
