@@ -301,6 +301,12 @@ int trb_base_gemm(const void* x, const void* base_weight, void* y, int num_token
 int trb_sgmv_stacked(void* y, const void* x, const void* w, const void* s, int num_problems, int num_rows,
                      int d_in, int d_out, int max_rows, int accumulate, int dtype, int dev, void* stream);
 
+/* trb_base_gemm (without LoRA operands) followed by trb_lora_indexed on the same y, x and shapes, the shrink of the
+ * second overlapping the first: y[t] = x[t] @ base_weight^T + scale * (x[t] @ wa[id]) @ wb[id]. */
+int trb_base_lora(const void* x, const void* base_weight, void* y, const void* wa, const void* wb, const void* indices,
+                  int index_is_64bit, int num_tokens, int prob_m, int prob_k, int rank, int num_adapters, float scale,
+                  int dtype, int dev, void* stream);
+
 /* Segment offsets of adapter ids for the segmented LoRA products: s[i] = number of ids in [-1, i) for i = 0 ..
  * num_adapters (int32 [num_adapters + 1]; ids outside [-1, num_adapters) are not counted).  The device form of the
  * host loop of triteia/python/ops/matmul/lora.py:63-78.  num_adapters <= 8191. */

@@ -1017,3 +1017,23 @@ def test_segment_offsets(cuda, T, M):
     for dtype in (torch.int32, torch.int64):
         ids = torch.from_numpy(np.sort(np.random.default_rng(T).integers(-3, M + 2, T))).to(dtype)
         assert torch.equal(segment_offsets(ids.to(cuda), M).cpu(), segment_offsets(ids, M))
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("K,N,rank", [(64, 8, 8), (320, 264, 24), (1024, 4104, 64)])
+def test_lora_bgmv_with_base(cuda, K, N, rank, dtype):
+    """lora_bgmv on a base weight (the shrink overlaps the base product): ranks whose pieces do not fill a warp's
+    groups, fewer and more output columns than the CTA covers at once, ids without an adapter on both sides, both
+    index types.  Against the oracle's lora statement; base and sum are each rounded once to the type."""
+    ops = _ops()
+    A, B, x, idx = lora_inputs(37, 5, K, N, rank, seed=rank, dtype=dtype)
+    idx[5], idx[11] = -1, 7
+    w = (torch.randn(N, K, device=cuda, generator=torch.Generator(cuda).manual_seed(1)) * 0.05).to(dtype)
+    idx_np = idx.cpu().numpy().copy()
+    idx_np[idx_np >= 5] = -1
+    ref = oracle.lora(A.float().cpu().numpy(), B.float().cpu().numpy(), x.float().cpu().numpy(), idx_np,
+                      base_weight=w.float().cpu().numpy(), scale=0.5)
+    for i in (idx, idx.long()):
+        y = ops.lora_bgmv(A, B, x, i, base_weight=w, scale=0.5)
+        assert oracle.row_rel_err(y.float().cpu().numpy(), ref).max() <= (ROW_TOL if dtype == torch.float16 else 3e-2)
+    assert _lib().device_status(0) == 0

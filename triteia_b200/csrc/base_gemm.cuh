@@ -183,7 +183,6 @@ base_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
   const int warp = tid >> 5;
   const int lane = tid & 31;
 
-  pdl_launch_dependents();
   if (tid == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full_bar[s], 1);
@@ -204,6 +203,8 @@ base_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   pdl_wait();   // x and V may come from the kernels launched just before
+  // Only now may the next kernel start: the indexed LoRA kernel reads its inputs without waiting for this one.
+  pdl_launch_dependents();
   const int n_seg = a.seg != nullptr ? max(0, min(a.n_seg, kMaxSegments)) : 0;
   if (a.seg != nullptr && warp == 0) {   // token tiles before each segment
     int running = 0;
@@ -753,6 +754,16 @@ extern "C" int trb_base_gemm(const void* x, const void* base_weight, void* y, in
   if (cudaSetDevice(dev) != cudaSuccess) return TRB_ERR_CUDA;
   return base_gemm_launch(x, base_weight, y, num_tokens, prob_m, prob_k, lora_v, lora_b, lora_k, accumulate ? 1 : 0,
                           dtype == TRB_BF16, dev, (cudaStream_t)stream);
+}
+
+extern "C" int trb_base_lora(const void* x, const void* base_weight, void* y, const void* wa, const void* wb,
+                             const void* indices, int index_is_64bit, int num_tokens, int prob_m, int prob_k, int rank,
+                             int num_adapters, float scale, int dtype, int dev, void* stream) {
+  using namespace trb;
+  const int r = trb_base_gemm(x, base_weight, y, num_tokens, prob_m, prob_k, nullptr, nullptr, 0, 0, dtype, dev, stream);
+  if (r != TRB_OK) return r;
+  return lora_indexed_call(y, x, wa, wb, indices, index_is_64bit, num_tokens, prob_k, prob_m, rank, num_adapters, scale, dtype,
+                           dev, 1, (cudaStream_t)stream);
 }
 
 extern "C" int trb_sgmv_stacked(void* y, const void* x, const void* w, const void* s, int num_problems, int num_rows,

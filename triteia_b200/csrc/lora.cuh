@@ -134,82 +134,152 @@ __global__ void __launch_bounds__(256) lora_fused_kernel(T* __restrict__ Y, cons
 
 // ---- indexed LoRA on the natural layouts A [M, h1, r], B [M, r, h2]: one CTA per token ----
 // The id space may be shared with deltas: ids outside [0, num_adapters) are skipped.
+// Bound by latency: a token reads (h1 + h2) * r values of its adapter (256 KiB at 2048 x 2048, r = 32), mostly from
+// L2, through one CTA.  16 warps with eight independent 16-byte loads per lane in flight; the lanes of a warp share
+// rows of A, so a load covers contiguous memory and a lane keeps 8 accumulators; the expand splits the rank over two
+// halves of the CTA.  100 tokens, 2048 -> 2048, r = 32: 16.0 us with 8 warps, a whole row of A per lane (64
+// accumulators) and the rank in sequence.
+// late_wait: everything this kernel reads but y was complete before the kernel launched just before could start
+// (base_gemm_kernel lets its successor start only after its own wait), so the shrink overlaps that kernel.
+constexpr int kLoraThreads = 512;
+
 template <class T, class IdxT>
-__global__ void __launch_bounds__(256) lora_indexed_kernel(T* __restrict__ Y, const T* __restrict__ X,
-                                                           const T* __restrict__ A, const T* __restrict__ B,
-                                                           const IdxT* __restrict__ indices, int h1, int h2, int rank,
-                                                           int num_adapters, float scale) {
-  __shared__ float part[8][64];
+__global__ void __launch_bounds__(kLoraThreads) lora_indexed_kernel(T* __restrict__ Y, const T* __restrict__ X,
+                                                                    const T* __restrict__ A, const T* __restrict__ B,
+                                                                    const IdxT* __restrict__ indices, int h1, int h2,
+                                                                    int rank, int num_adapters, float scale,
+                                                                    int late_wait) {
+  constexpr int WARPS = kLoraThreads / 32, HALF = kLoraThreads / 2;
+  __shared__ float part[WARPS][64];
   __shared__ float v[64];
+  __shared__ float4 upper[2][HALF];      // the upper rank half's sums of 8 output features per thread
+  pdl_launch_dependents();
+  if (!late_wait) pdl_wait();
   const int b = blockIdx.x;
   const long long idx = (long long)indices[b];
-  if (idx < 0 || idx >= num_adapters) return;
+  if (idx < 0 || idx >= num_adapters) {
+    if (late_wait) pdl_wait();
+    return;
+  }
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const T* a = A + idx * (int64_t)h1 * rank;
   const T* x = X + (int64_t)b * h1;
-  float acc[64];
-#pragma unroll
-  for (int j = 0; j < 64; ++j) acc[j] = 0.f;
+  // A row of A holds rank values = rv 16-byte pieces; `pw` lanes (rv rounded up to a power of two) share a row.
   const int rv = rank / 8;
-  for (int k = tid; k < h1; k += 256) {
-    const float xk = Cvt<T>::to_f(x[k]);
-    const uint4* row = reinterpret_cast<const uint4*>(a + (int64_t)k * rank);
+  const int pw = rv <= 1 ? 1 : (rv <= 2 ? 2 : (rv <= 4 ? 4 : 8));
+  const int sub = lane & (pw - 1), rl = lane / pw, rows_per_warp = 32 / pw;
+  float acc[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      if (i < rv) {
-        const uint4 wv = row[i];
-        const uint32_t* pw = reinterpret_cast<const uint32_t*>(&wv);
+  for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+  if (sub < rv) {
+#pragma unroll 8
+    for (int k = warp * rows_per_warp + rl; k < h1; k += WARPS * rows_per_warp) {
+      const float xk = Cvt<T>::to_f(x[k]);
+      const uint4 wv = *reinterpret_cast<const uint4*>(a + (int64_t)k * rank + sub * 8);
+      const uint32_t* pwv = reinterpret_cast<const uint32_t*>(&wv);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 f = Cvt<T>::to_f2(pw[e]);
-          acc[i * 8 + 2 * e] = fmaf(xk, f.x, acc[i * 8 + 2 * e]);
-          acc[i * 8 + 2 * e + 1] = fmaf(xk, f.y, acc[i * 8 + 2 * e + 1]);
-        }
+      for (int e = 0; e < 4; ++e) {
+        const float2 f = Cvt<T>::to_f2(pwv[e]);
+        acc[2 * e] = fmaf(xk, f.x, acc[2 * e]);
+        acc[2 * e + 1] = fmaf(xk, f.y, acc[2 * e + 1]);
       }
     }
   }
+  for (int o = pw; o < 32; o <<= 1)
 #pragma unroll
-  for (int j = 0; j < 64; ++j) {
-    if (j < rank) {
-      const float s = warp_sum(acc[j]);
-      if (lane == 0) part[warp][j] = s;
-    }
-  }
+    for (int e = 0; e < 8; ++e) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
+  if (lane < pw && sub < rv)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) part[warp][sub * 8 + e] = acc[e];
   __syncthreads();
   if (tid < rank) {
     float s = 0.f;
 #pragma unroll
-    for (int w = 0; w < 8; ++w) s += part[w][tid];
+    for (int w = 0; w < WARPS; ++w) s += part[w][tid];
     v[tid] = s * scale;
   }
   __syncthreads();
+  if (late_wait) pdl_wait();             // y comes from the kernel before
   const T* bm = B + idx * (int64_t)rank * h2;
-  for (int o8 = tid; o8 < h2 / 8; o8 += 256) {
+  const int col = tid & (HALF - 1), top = tid / HALF;
+  const int j0 = top * (rank / 2), j1 = j0 + rank / 2;
+  for (int base = 0; base < h2 / 8; base += HALF) {
+    const int o8 = base + col;
     float out[8];
-    const uint4 yv = *reinterpret_cast<const uint4*>(Y + (int64_t)b * h2 + o8 * 8);
-    const uint32_t* py = reinterpret_cast<const uint32_t*>(&yv);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float2 f = Cvt<T>::to_f2(py[e]);
-      out[2 * e] = f.x;
-      out[2 * e + 1] = f.y;
-    }
-    for (int j = 0; j < rank; ++j) {
-      const uint4 wv = *reinterpret_cast<const uint4*>(bm + (int64_t)j * h2 + o8 * 8);
-      const uint32_t* pw = reinterpret_cast<const uint32_t*>(&wv);
-      const float vj = v[j];
+    for (int e = 0; e < 8; ++e) out[e] = 0.f;
+    if (o8 < h2 / 8) {
+#pragma unroll 8
+      for (int j = j0; j < j1; ++j) {
+        const uint4 wv = *reinterpret_cast<const uint4*>(bm + (int64_t)j * h2 + o8 * 8);
+        const uint32_t* pw32 = reinterpret_cast<const uint32_t*>(&wv);
+        const float vj = v[j];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 f = Cvt<T>::to_f2(pw[e]);
-        out[2 * e] = fmaf(vj, f.x, out[2 * e]);
-        out[2 * e + 1] = fmaf(vj, f.y, out[2 * e + 1]);
+        for (int e = 0; e < 4; ++e) {
+          const float2 f = Cvt<T>::to_f2(pw32[e]);
+          out[2 * e] = fmaf(vj, f.x, out[2 * e]);
+          out[2 * e + 1] = fmaf(vj, f.y, out[2 * e + 1]);
+        }
       }
     }
-    T o[8];
+    if (top == 1) {
+      upper[0][col] = make_float4(out[0], out[1], out[2], out[3]);
+      upper[1][col] = make_float4(out[4], out[5], out[6], out[7]);
+    }
+    __syncthreads();
+    if (top == 0 && o8 < h2 / 8) {
+      uint4* yp = reinterpret_cast<uint4*>(Y + (int64_t)b * h2 + o8 * 8);
+      const uint4 yv = *yp;
+      const uint32_t* py = reinterpret_cast<const uint32_t*>(&yv);
+      const float4 u0 = upper[0][col], u1 = upper[1][col];
+      const float up[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+      T o[8];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) o[e] = Cvt<T>::from_f(out[e]);
-    *reinterpret_cast<uint4*>(Y + (int64_t)b * h2 + o8 * 8) = *reinterpret_cast<uint4*>(o);
+      for (int e = 0; e < 4; ++e) {
+        const float2 f = Cvt<T>::to_f2(py[e]);
+        o[2 * e] = Cvt<T>::from_f(f.x + (out[2 * e] + up[2 * e]));
+        o[2 * e + 1] = Cvt<T>::from_f(f.y + (out[2 * e + 1] + up[2 * e + 1]));
+      }
+      *yp = *reinterpret_cast<uint4*>(o);
+    }
+    __syncthreads();                     // `upper` is written again for the next columns
   }
+}
+
+template <class T, class IdxT>
+static int lora_indexed_launch(void* y, const void* x, const void* wa, const void* wb, const void* indices, int batch, int h1,
+                               int h2, int rank, int num_adapters, float scale, int late_wait, cudaStream_t stream) {
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(batch);
+  lc.blockDim = dim3(kLoraThreads);
+  lc.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = at;
+  lc.numAttrs = 1;
+  return cudaLaunchKernelEx(&lc, lora_indexed_kernel<T, IdxT>, (T*)y, (const T*)x, (const T*)wa, (const T*)wb,
+                            (const IdxT*)indices, h1, h2, rank, num_adapters, scale, late_wait) == cudaSuccess
+             ? TRB_OK
+             : TRB_ERR_CUDA;
+}
+
+// Argument checks and choice of the instantiation.  late_wait: see the kernel.
+static int lora_indexed_call(void* y, const void* x, const void* wa, const void* wb, const void* indices,
+                             int index_is_64bit, int batch, int h1, int h2, int rank, int num_adapters, float scale,
+                             int dtype, int dev, int late_wait, cudaStream_t st) {
+  if (batch == 0 || num_adapters == 0) return TRB_OK;
+  if (batch < 0 || num_adapters < 0 || !y || !x || !wa || !wb || !indices) return TRB_ERR_BAD_ARG;
+  if (rank <= 0 || rank > 64 || rank % 8 != 0 || h1 <= 0 || h2 <= 0 || h2 % 8 != 0) return TRB_ERR_KERN_SHAPE;
+  if (((uintptr_t)y | (uintptr_t)wa | (uintptr_t)wb) & 15) return TRB_ERR_BAD_ARG;
+  if (cudaSetDevice(dev) != cudaSuccess) return TRB_ERR_CUDA;
+  if (dtype == TRB_F16)
+    return index_is_64bit ? lora_indexed_launch<__half, int64_t>(y, x, wa, wb, indices, batch, h1, h2, rank, num_adapters, scale, late_wait, st)
+                          : lora_indexed_launch<__half, int32_t>(y, x, wa, wb, indices, batch, h1, h2, rank, num_adapters, scale, late_wait, st);
+  if (dtype == TRB_BF16)
+    return index_is_64bit ? lora_indexed_launch<__nv_bfloat16, int64_t>(y, x, wa, wb, indices, batch, h1, h2, rank, num_adapters, scale, late_wait, st)
+                          : lora_indexed_launch<__nv_bfloat16, int32_t>(y, x, wa, wb, indices, batch, h1, h2, rank, num_adapters, scale, late_wait, st);
+  return TRB_ERR_KERN_SHAPE;
 }
 
 // ---- SGMV: y[seg] += x[seg] @ W_seg, 64-token x BN-column tiles on mma.sync m16n8k16 ----
@@ -454,23 +524,6 @@ extern "C" int trb_sgmv(void* y, const void* x, const void* w, const void* s, vo
 extern "C" int trb_lora_indexed(void* y, const void* x, const void* wa, const void* wb, const void* indices,
                                 int index_is_64bit, int batch, int h1, int h2, int rank, int num_adapters,
                                 float scale, int dtype, int dev, void* stream) {
-  using namespace trb;
-  if (batch == 0 || num_adapters == 0) return TRB_OK;
-  if (batch < 0 || num_adapters < 0 || !y || !x || !wa || !wb || !indices) return TRB_ERR_BAD_ARG;
-  if (rank <= 0 || rank > 64 || rank % 8 != 0 || h1 <= 0 || h2 <= 0 || h2 % 8 != 0) return TRB_ERR_KERN_SHAPE;
-  if (((uintptr_t)y | (uintptr_t)wa | (uintptr_t)wb) & 15) return TRB_ERR_BAD_ARG;
-  if (cudaSetDevice(dev) != cudaSuccess) return TRB_ERR_CUDA;
-  cudaStream_t st = (cudaStream_t)stream;
-#define TRB_LORA_IDX(T, I)                                                                                        \
-  lora_indexed_kernel<T, I><<<batch, 256, 0, st>>>((T*)y, (const T*)x, (const T*)wa, (const T*)wb, (const I*)indices, \
-                                                   h1, h2, rank, num_adapters, scale)
-  if (dtype == TRB_F16) {
-    if (index_is_64bit) TRB_LORA_IDX(__half, int64_t); else TRB_LORA_IDX(__half, int32_t);
-  } else if (dtype == TRB_BF16) {
-    if (index_is_64bit) TRB_LORA_IDX(__nv_bfloat16, int64_t); else TRB_LORA_IDX(__nv_bfloat16, int32_t);
-  } else {
-    return TRB_ERR_KERN_SHAPE;
-  }
-#undef TRB_LORA_IDX
-  return cudaGetLastError() == cudaSuccess ? TRB_OK : TRB_ERR_CUDA;
+  return trb::lora_indexed_call(y, x, wa, wb, indices, index_is_64bit, batch, h1, h2, rank, num_adapters, scale, dtype, dev, 0,
+                                (cudaStream_t)stream);
 }

@@ -42,7 +42,20 @@ def lora_indexed(y, x, weights_A, weights_B, indices, scale=1.0):
 def lora_bgmv(weights_A, weights_B, x, indices, base_weight=None, layer_idx=0, scale=1.0):
     """One adapter per token.  One launch on the natural layouts: no per-call transpose of the
     adapters, no gather / scatter of the rows (compare lora.py:33-47 of the reference)."""
-    y = _base(x, base_weight, weights_B.shape[2])
+    M, K, rank = weights_A.shape
+    N = weights_B.shape[2]
+    if (base_weight is not None and x.is_cuda and base_weight.dtype == x.dtype and tuple(base_weight.shape) == (N, K)
+            and x.shape[1] == K and rank % 8 == 0 and 0 < rank <= 64 and K % 64 == 0 and N % 8 == 0 and M > 0):
+        # one call: the shrink overlaps the base product
+        weights_A, weights_B, x, base_weight = (t.contiguous() for t in (weights_A, weights_B, x, base_weight))
+        if indices.dtype not in (torch.int32, torch.int64):
+            indices = indices.to(torch.int32)
+        y = torch.empty(x.shape[0], N, dtype=x.dtype, device=x.device)
+        _lib.check(lib.trb_base_lora(ptr(x), ptr(base_weight), ptr(y), ptr(weights_A), ptr(weights_B), ptr(indices),
+                                     int(indices.dtype == torch.int64), x.shape[0], N, K, rank, M, float(scale),
+                                     _lib.dtype_tag(x.dtype), dev_of(x), stream_of(x)), "base_lora")
+        return y
+    y = _base(x, base_weight, N)
     if not (weights_A.is_contiguous() and weights_B.is_contiguous() and x.is_contiguous()):
         weights_A, weights_B, x = weights_A.contiguous(), weights_B.contiguous(), x.contiguous()
     return lora_indexed(y, x, weights_A, weights_B, indices, scale)
