@@ -287,6 +287,19 @@ int trb_base_gemm(const void* x, const void* base_weight, void* y, int num_token
                   const void* lora_v, const void* lora_b, int lora_k, int accumulate, int dtype, int dev,
                   void* stream);
 
+/* Base product plus, per token, a LoRA adapter or a packed delta, in one call (ldmm, and with
+ * num_adapters = 0 the base-weight form of sbmm):
+ *   y[t] = x[t] @ base_weight^T + (x[t] @ wa[id]) @ wb[id]         0 <= id < num_adapters
+ *   y[t] = x[t] @ base_weight^T + x[t] @ delta[id - num_adapters]  num_adapters <= id < num_adapters + num_deltas
+ * and the base product alone for any other id (triteia/python/ops/matmul/ldmm.py:51-107, sbmm.py:89-123).
+ * fp16, indices int32; wa [num_adapters, K, rank], wb [num_adapters, rank, N], rank <= 64 and a multiple of
+ * 8; shapes otherwise as trb_base_gemm and trb_sbmm_indexed.  v [T, num_adapters * rank] fp16 (the shrink's
+ * result; NULL without adapters) and scratch (as trb_sbmm_indexed) are working memory. */
+int trb_base_indexed(const void* x, const void* base_weight, const void* wa, const void* wb, const void* qweights,
+                     const void* metas, const void* scales, const void* indices, void* y, void* v, int num_tokens,
+                     int prob_m, int prob_k, int num_adapters, int rank, int num_deltas, int groupsize, void* scratch,
+                     size_t scratch_bytes, int dev, void* stream);
+
 /* SGMV on a stacked weight tensor, on the tcgen05 tensor cores:
  *   y[s[i] : s[i + 1], :] (+)= x[s[i] : s[i + 1], :] @ w[i],   i < num_problems,
  * x [num_rows, d_in], y [num_rows, d_out], w [num_problems, d_in, d_out] row-major (the layout of the

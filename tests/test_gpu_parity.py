@@ -1037,3 +1037,39 @@ def test_lora_bgmv_with_base(cuda, K, N, rank, dtype):
         y = ops.lora_bgmv(A, B, x, i, base_weight=w, scale=0.5)
         assert oracle.row_rel_err(y.float().cpu().numpy(), ref).max() <= (ROW_TOL if dtype == torch.float16 else 3e-2)
     assert _lib().device_status(0) == 0
+
+
+@pytest.mark.parametrize("base_only", [False, True])
+def test_fused_calls_follow_what_produced_their_inputs(cuda, base_only):
+    """The one-call forms of ldmm and of sbmm with a base weight, whose kernels overlap each other, started right
+    behind kernels that produce x and the ids and let their successors start early: the same bits as with a
+    synchronisation before and after every call."""
+    ops = _ops()
+    K = N = 1024
+    T, D, M = 96, 12, 6
+    qs, metas, ss = packed(N, K, 128, seed=2, num=D)
+    g = torch.Generator(cuda).manual_seed(4)
+    w = (torch.randn(N, K, device=cuda, generator=g) * 0.02).half()
+    A = (torch.randn(M, K, 16, device=cuda, generator=g) / 32).half()
+    B = (torch.randn(M, 16, N, device=cuda, generator=g) / 4).half()
+    ids0 = torch.from_numpy(np.random.default_rng(0).integers(-1, D if base_only else M + D, T).astype(np.int32)).to(cuda)
+    x0 = torch.randn(T, K, device=cuda, generator=g).half()
+
+    def run(sync):
+        x, out = x0, []
+        for i in range(12):
+            if sync:
+                torch.cuda.synchronize()
+            z = ops.matmul_4bit_2_4(qs[i % D], x, metas[i % D], ss[i % D])
+            ids = torch.roll(ids0, i)
+            if sync:
+                torch.cuda.synchronize()
+            y = (ops.sbmm_4bit_2_4_native(qs, z, metas, ss, ids, base_weight=w) if base_only
+                 else ops.ldmm(ids, z, A, B, qs, metas, ss, base_weight=w))
+            x = (y / y.float().std()).half()
+            out.append(y)
+        return out
+
+    a, b = run(True), run(False)
+    assert all(torch.equal(p, q) for p, q in zip(a, b))
+    assert _lib().device_status(0) == 0

@@ -53,6 +53,7 @@ SIGNATURES = {
     "trb_base_gemm": (_i, [_vp] * 3 + [_i] * 3 + [_vp, _vp] + [_i] * 4 + [_vp]),
     "trb_segments": (_i, [_vp] + [_i] * 3 + [_vp, _i, _vp]),
     "trb_base_lora": (_i, [_vp] * 6 + [_i] * 6 + [_f, _i, _i, _vp]),
+    "trb_base_indexed": (_i, [_vp] * 10 + [_i] * 7 + [_vp, _sz, _i, _vp]),
     "trb_sgmv_stacked": (_i, [_vp] * 4 + [_i] * 8 + [_vp]),
     "trb_lora_shrink_rows": (_i, [_vp] * 4 + [_i] * 6 + [_f, _i, _vp]),
     "trb_sgmv_tmp_size": (_sz, [_i]),
@@ -83,13 +84,13 @@ def ptr(t):
 
 
 def stream_of(t):
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(dev_of(t))
 
 
 def dev_of(t):
     if not t.is_cuda:
         raise RuntimeError("triteia_b200: tensors must live on a CUDA device (there is no CPU path)")
-    return t.device.index if t.device.index is not None else torch.cuda.current_device()
+    return t.get_device()
 
 
 def status_string(code):

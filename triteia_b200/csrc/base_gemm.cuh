@@ -54,6 +54,7 @@ struct BaseArgs {
   __half* y;          // fp16 or bf16 by `bf16`
   int accumulate;     // y += result instead of y = result
   int bf16;           // operands and output are bfloat16
+  int late_wait;      // the kernel just before feeds a later one only: wait for it at the end (see lora_shrink_rows_kernel)
   // Segmented form (seg != nullptr), the SGMV of the LoRA operators: rows [seg[i], seg[i + 1]) of the
   // input [T, seg_k] meet weight i of a stacked tensor [n_seg, seg_k, N] (row-major, so an MN-major
   // operand as it lies in memory).  K is unused, x is the input, the stacked weights come through tm_b.
@@ -202,7 +203,7 @@ base_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
-  pdl_wait();   // x and V may come from the kernels launched just before
+  if (!a.late_wait) pdl_wait();   // x and V may come from the kernels launched just before
   // Only now may the next kernel start: the indexed LoRA kernel reads its inputs without waiting for this one.
   pdl_launch_dependents();
   const int n_seg = a.seg != nullptr ? max(0, min(a.n_seg, kMaxSegments)) : 0;
@@ -533,6 +534,7 @@ base_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
     }
   }
 
+  if (a.late_wait) pdl_wait();
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();   // no CTA leaves, or frees TMEM, while another may still touch it
@@ -546,17 +548,22 @@ base_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
 // in [0, num_adapters); the row stays zero for any other id.  One CTA per token, A [M, h1, rank] in
 // its natural layout.  This is the shrink half of the reference's BGMV pair
 // (triteia/csrc/ops/bgmv_impl.cuh:15-137) writing straight into the operand of the expand above.
+// late_wait: the kernel launched just before (the row gather of a fused call) writes nothing this one reads, and it
+// started only after everything that does had finished, so the two overlap; this one still ends after it, which
+// keeps the order of the stream for the kernels behind.
 constexpr int kShrinkThreads = 512;
 
 template <class IdxT>
 __global__ void __launch_bounds__(kShrinkThreads) lora_shrink_rows_kernel(__half* __restrict__ V, const __half* __restrict__ X,
                                                                const __half* __restrict__ A,
                                                                const IdxT* __restrict__ indices, int h1, int rank,
-                                                               int num_adapters, int v_cols, float scale) {
+                                                               int num_adapters, int v_cols, float scale,
+                                                               int late_wait) {
   constexpr int WARPS = kShrinkThreads / 32;
   __shared__ float part[WARPS][64];
   const int b = blockIdx.x;
   pdl_launch_dependents();
+  if (!late_wait) pdl_wait();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   uint4* vrow = reinterpret_cast<uint4*>(V + (int64_t)b * v_cols);
   const long long idx = (long long)indices[b];
@@ -564,7 +571,10 @@ __global__ void __launch_bounds__(kShrinkThreads) lora_shrink_rows_kernel(__half
   const int lo8 = has ? (int)idx * rank / 8 : -1, hi8 = has ? lo8 + rank / 8 : -1;
   for (int i = tid; i < v_cols / 8; i += kShrinkThreads)
     if (i < lo8 || i >= hi8) vrow[i] = make_uint4(0, 0, 0, 0);
-  if (!has) return;
+  if (!has) {
+    if (late_wait) pdl_wait();
+    return;
+  }
   const __half* am = A + idx * (int64_t)h1 * rank;
   const __half* x = X + (int64_t)b * h1;
   // A row of A holds rank halves = rv 16-byte pieces.  `pw` lanes (rv rounded up to a power of two)
@@ -604,6 +614,7 @@ __global__ void __launch_bounds__(kShrinkThreads) lora_shrink_rows_kernel(__half
     for (int w = 0; w < WARPS; ++w) s += part[w][tid];
     V[(int64_t)b * v_cols + idx * rank + tid] = __float2half_rn(s * scale);
   }
+  if (late_wait) pdl_wait();
 }
 
 static_assert(BaseCfg::SMEM_ALLOC <= 232448, "shared memory budget of one sm_100 CTA");
@@ -684,8 +695,9 @@ static int base_gemm_launch_args(BaseArgs a, const CUtensorMap& tx, const CUtens
 static int token_tile_for(int rows) { return rows <= 32 ? 32 : rows <= 64 ? 64 : rows <= 128 ? 128 : 256; }
 
 static int base_gemm_launch(const void* x, const void* w, void* y, int T, int N, int K, const void* v, const void* b,
-                            int kv, int accumulate, int bf16, int dev, cudaStream_t stream) {
+                            int kv, int accumulate, int bf16, int dev, cudaStream_t stream, int late_wait = 0) {
   BaseArgs a{};
+  a.late_wait = late_wait;
   a.T = T; a.N = N; a.K = K; a.kv = kv;
   a.tt = token_tile_for(T);
   a.group = kTileGroup;
@@ -736,6 +748,24 @@ static int sgmv_stacked_launch(void* y, const void* x, const void* w, const int*
     return TRB_ERR_CUDA;
   const long long items = ((long long)T / a.tt + n_seg) * ((d_out + 255) / 256);     // upper bound: the lengths are on the device
   return base_gemm_launch_args(a, tx, tx, tx, tb, items, dev, stream);
+}
+
+template <class IdxT>
+static int lora_shrink_rows_launch(void* v, const void* x, const void* wa, const void* indices, int batch, int h1, int rank,
+                                   int num_adapters, int v_cols, float scale, int late_wait, cudaStream_t stream) {
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(batch);
+  lc.blockDim = dim3(kShrinkThreads);
+  lc.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = at;
+  lc.numAttrs = 1;
+  return cudaLaunchKernelEx(&lc, lora_shrink_rows_kernel<IdxT>, (__half*)v, (const __half*)x, (const __half*)wa,
+                            (const IdxT*)indices, h1, rank, num_adapters, v_cols, scale, late_wait) == cudaSuccess
+             ? TRB_OK
+             : TRB_ERR_CUDA;
 }
 
 }  // namespace trb
@@ -791,11 +821,41 @@ extern "C" int trb_lora_shrink_rows(void* v, const void* x, const void* wa, cons
   if (((uintptr_t)v | (uintptr_t)wa) & 15) return TRB_ERR_BAD_ARG;
   if (cudaSetDevice(dev) != cudaSuccess) return TRB_ERR_CUDA;
   cudaStream_t st = (cudaStream_t)stream;
-  if (index_is_64bit)
-    lora_shrink_rows_kernel<int64_t><<<batch, kShrinkThreads, 0, st>>>((__half*)v, (const __half*)x, (const __half*)wa,
-                                                            (const int64_t*)indices, h1, rank, num_adapters, v_cols, scale);
-  else
-    lora_shrink_rows_kernel<int32_t><<<batch, kShrinkThreads, 0, st>>>((__half*)v, (const __half*)x, (const __half*)wa,
-                                                            (const int32_t*)indices, h1, rank, num_adapters, v_cols, scale);
-  return cudaGetLastError() == cudaSuccess ? TRB_OK : TRB_ERR_CUDA;
+  return index_is_64bit
+             ? lora_shrink_rows_launch<int64_t>(v, x, wa, indices, batch, h1, rank, num_adapters, v_cols, scale, 0, st)
+             : lora_shrink_rows_launch<int32_t>(v, x, wa, indices, batch, h1, rank, num_adapters, v_cols, scale, 0, st);
+}
+
+// One call for base product + (LoRA adapter or packed delta) per token: router and row gather of the delta part
+// first, the LoRA shrink (or, without adapters, the base product) overlapping them, then base product and LoRA
+// expand into y, then the grouped delta kernels adding into y.  The order lets the small kernels run beside the large
+// ones on one stream, without a second stream, events or a host call per kernel.
+extern "C" int trb_base_indexed(const void* x, const void* base_weight, const void* wa, const void* wb, const void* qweights,
+                                const void* metas, const void* scales, const void* indices, void* y, void* v, int num_tokens,
+                                int prob_m, int prob_k, int num_adapters, int rank, int num_deltas, int groupsize,
+                                void* scratch, size_t scratch_bytes, int dev, void* stream_v) {
+  using namespace trb;
+  if (num_tokens < 0 || prob_m < 0 || prob_k < 0 || num_adapters < 0 || num_deltas <= 0) return TRB_ERR_BAD_ARG;
+  if (num_tokens == 0 || prob_m == 0) return TRB_OK;
+  if (!x || !base_weight || !y || !indices || !scratch || (num_adapters > 0 && (!wa || !wb || !v))) return TRB_ERR_BAD_ARG;
+  if (prob_k == 0 || prob_k % 64 != 0 || prob_m % 8 != 0) return TRB_ERR_PROB_SHAPE;
+  if (num_adapters > 0 && (rank <= 0 || rank > 64 || rank % 8 != 0)) return TRB_ERR_KERN_SHAPE;
+  if (((uintptr_t)x | (uintptr_t)base_weight | (uintptr_t)y | (uintptr_t)wa | (uintptr_t)wb | (uintptr_t)v) & 15) return TRB_ERR_BAD_ARG;
+  const int v_cols = num_adapters * rank;
+  cudaStream_t stream = (cudaStream_t)stream_v;
+  RouteSrc src{};
+  src.indices = (const int*)indices;
+  src.id_offset = num_adapters;
+  auto delta = [&](int phase) {
+    return sbmm_indexed_impl(x, qweights, metas, scales, src, y, num_tokens, prob_m, prob_k, num_deltas, groupsize, 1, scratch,
+                             scratch_bytes, dev, stream, nullptr, 0, phase);
+  };
+  int r = delta(1);
+  if (r == TRB_OK && num_adapters > 0)
+    r = lora_shrink_rows_launch<int32_t>(v, x, wa, indices, num_tokens, prob_k, rank, num_adapters, v_cols, 1.f, 1, stream);
+  if (r == TRB_OK)
+    r = base_gemm_launch(x, base_weight, y, num_tokens, prob_m, prob_k, num_adapters > 0 ? v : nullptr,
+                         num_adapters > 0 ? wb : nullptr, v_cols, 0, 0, dev, stream, num_adapters > 0 ? 0 : 1);
+  if (r == TRB_OK) r = delta(2);
+  return r;
 }

@@ -108,7 +108,6 @@ route_kernel(const RouteSrc src, int T, int D, int W, int TT, int* __restrict__ 
              int* __restrict__ counters, int* __restrict__ slot_of, int slot_stride, int* __restrict__ bin_count,
              const RouteClasses cl) {
   extern __shared__ int sm[];
-  pdl_launch_dependents();
   const int bins = D + 1;             // bin 0 = id -1 (and out-of-range ids)
   int* hist = sm;                     // [bins][W]
   int* bin_start = hist + bins * W;   // [bins + 1]
@@ -123,8 +122,11 @@ route_kernel(const RouteSrc src, int T, int D, int W, int TT, int* __restrict__ 
   if (tid == 0) n_invalid = 0;
   __syncthreads();
   // Launched with programmatic stream serialization: everything above overlaps the tail of the kernel
-  // before; the ids may come from it and the outputs may still be read by it, so wait here.
+  // before; the ids may come from it and the outputs may still be read by it, so wait here.  Only then may
+  // the next kernel start: what follows the gather (the LoRA shrink or the base product of a fused call) reads
+  // its inputs without a wait of its own, because everything before the router has finished by then.
   pdl_wait();
+  pdl_launch_dependents();
 
   const int piece = ((T + W - 1) / W + 31) / 32 * 32;   // tokens per warp, multiple of 32
   const int t_lo = warp * piece, t_hi = min(T, t_lo + piece);

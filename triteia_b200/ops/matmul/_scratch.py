@@ -16,7 +16,7 @@ def scratch(device, nbytes, stream=None):
     current stream of the device), 256-byte aligned, reused by later calls on the same stream."""
     index = device.index if device.index is not None else torch.cuda.current_device()
     if stream is None:
-        stream = torch.cuda.current_stream(device).cuda_stream
+        stream = torch._C._cuda_getCurrentRawStream(index)
     key = (index, int(stream))
     buf = _buffers.get(key)
     if buf is None or buf.numel() < nbytes:

@@ -85,39 +85,36 @@ def sbmm_indexed(xs, qweights, metas, ss, indices, y=None, index_offset=0):
     return y
 
 
-class IndexedDeltaCall:
-    """`sbmm_indexed(..., y=y)` in two steps, so that the router and the row gather (`plan`, which
-    write nothing but the scratch) can run on another stream beside the kernel that produces y, and
-    the grouped kernels (`run`) after both.  The scratch belongs to the stream that is current at
-    construction; `plan` may be issued on any stream, the caller orders `run` after it."""
-
-    def __init__(self, xs, qweights, metas, ss, indices, y, index_offset=0):
-        T, K = xs.shape
-        D, G, N = ss.shape
-        if indices.dtype != torch.int32:
-            indices = indices.to(torch.int32)
-        self.t = (xs, qweights, metas, ss, indices, y)
-        self.dims = (T, N, K, D, int(index_offset), -1 if G == 1 else K // G)
-        self.buf = scratch(xs.device, lib.trb_sbmm_indexed_scratch_bytes(T, K, D))
-
-    def _call(self, phase):
-        xs, q, m, s, idx, y = self.t
-        T, N, K, D, off, groupsize = self.dims
-        err = lib.trb_sbmm_indexed_phase(ptr(xs), ptr(q), ptr(m), ptr(s), ptr(idx), ptr(y), T, N, K, D, off, groupsize,
-                                         1, ptr(self.buf), self.buf.numel(), phase, dev_of(xs), stream_of(xs))
-        _lib.check(err, "sbmm_indexed_phase")
-
-    def plan(self):
-        self._call(1)
-
-    def run(self):
-        self._call(2)
+def base_indexed(xs, base_weight, qweights, metas, ss, indices, weights_A=None, weights_B=None):
+    """One call: y = xs @ base_weight.t() plus each token's adapter (ids [0, M)) or delta (ids [M, M + D)); without
+    adapters M = 0.  fp16; weights_A [M, K, r], weights_B [M, r, N] contiguous."""
+    T, K = xs.shape
+    D, G, N = ss.shape
+    if base_weight.dtype != xs.dtype:
+        base_weight = base_weight.to(xs.dtype)
+    if not base_weight.is_contiguous():
+        base_weight = base_weight.contiguous()
+    if indices.dtype != torch.int32:
+        indices = indices.to(torch.int32)
+    M, rank = (0, 0) if weights_A is None else (weights_A.shape[0], weights_A.shape[2])
+    y = torch.empty(T, N, dtype=xs.dtype, device=xs.device)
+    v = torch.empty(T, M * rank, dtype=xs.dtype, device=xs.device) if M else None
+    buf = scratch(xs.device, lib.trb_sbmm_indexed_scratch_bytes(T, K, D))
+    err = lib.trb_base_indexed(ptr(xs), ptr(base_weight), ptr(weights_A), ptr(weights_B), ptr(qweights), ptr(metas), ptr(ss),
+                               ptr(indices), ptr(y), ptr(v), T, N, K, M, rank, D, -1 if G == 1 else K // G, ptr(buf), buf.numel(),
+                               dev_of(xs), stream_of(xs))
+    if err in (_lib.ERR_PROB_SHAPE, _lib.ERR_KERN_SHAPE):
+        raise RuntimeError(f"No suitable kernel. base product and deltas K={K} N={N} rank={rank} groups={G}")
+    _lib.check(err, "base_indexed")
+    return y
 
 
 def sbmm_4bit_2_4_native(qweights, xs, metas, ss, indices, base_weight=None):
     if not xs.is_contiguous():
         xs = xs.contiguous()
     if base_weight is not None:
+        if xs.dtype == torch.float16 and tuple(base_weight.shape) == (ss.shape[2], xs.shape[1]) and xs.shape[0] > 0:
+            return base_indexed(xs, base_weight, qweights, metas, ss, indices)
         y = base_gemm(xs, base_weight)
         return sbmm_indexed(xs, qweights, metas, ss, indices, y=y)
     return sbmm_indexed(xs, qweights, metas, ss, indices)

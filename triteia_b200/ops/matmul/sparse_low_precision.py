@@ -11,6 +11,5 @@ def matmul_4bit_2_4(qweight, x, meta, s):
     Returns fp16 [..., N].
     """
     C = torch.empty((x.shape[:-1] + (s.shape[1],)), dtype=x.dtype, device=x.device)
-    workspace = torch.zeros(s.shape[1], dtype=torch.int32, device=x.device)
-    mul_2_4(x.reshape(-1, x.shape[-1]), qweight, meta, C.view(-1, C.shape[-1]), s, workspace)
+    mul_2_4(x.reshape(-1, x.shape[-1]), qweight, meta, C.view(-1, C.shape[-1]), s, None)
     return C

@@ -46,7 +46,7 @@ def mul_2_4(A, B, meta, C, s, workspace, thread_k=-1, thread_m=-1, sms=-1, max_p
         _check_input(t, n)
     prob_n, prob_m, prob_k = A.size(0), C.size(1), A.size(1)
     groupsize = _group_arg(s.size(0), prob_k, "mul_2_4")
-    if workspace.numel() < prob_m // 128 * max_par:
+    if workspace is not None and workspace.numel() < prob_m // 128 * max_par:      # None: the kernel uses no workspace
         raise RuntimeError(f"workspace must be of size at least {prob_m // 128 * max_par}.")
     err = lib.trb_mul_2_4(ptr(A), ptr(B), ptr(meta), ptr(C), ptr(s), prob_m, prob_n, prob_k, ptr(workspace),
                           groupsize, dev_of(A), stream_of(A), thread_k, thread_m, sms, max_par)
