@@ -1073,3 +1073,22 @@ def test_fused_calls_follow_what_produced_their_inputs(cuda, base_only):
     a, b = run(True), run(False)
     assert all(torch.equal(p, q) for p, q in zip(a, b))
     assert _lib().device_status(0) == 0
+
+
+@pytest.mark.parametrize("T", [1, 31, 256, 257, 1024, 1025])
+@pytest.mark.parametrize("D", [1, 5, 300])
+def test_router_and_gather_in_one_launch(cuda, T, D):
+    """sbmm at the limits of the fused router and gather (its two block sizes, the longest batch, more bins than its
+    shared memory takes; one token past the limit uses two launches), ids in any order with some outside the range.
+    Every row against the oracle; rows without a delta are zero."""
+    ops = _ops()
+    qs, metas, ss = packed(128, 128, 128, seed=D, num=D)
+    rng = np.random.default_rng(T * 7 + D)
+    idx_np = rng.integers(-2, D + 2, T).astype(np.int32)
+    x = torch.randn(T, 128, dtype=torch.float16, device=cuda, generator=torch.Generator(cuda).manual_seed(T))
+    idx = torch.from_numpy(idx_np).to(cuda)
+    y = ops.sbmm_4bit_2_4_native(qs, x, metas, ss, idx)
+    none = (idx_np < 0) | (idx_np >= D)
+    clean = np.where(none, -1, idx_np).astype(np.int32)
+    check(y, oracle.sbmm(qs.cpu().numpy(), x.cpu().numpy(), metas.cpu().numpy(), ss.cpu().numpy(), clean), mean_tol=None)
+    assert torch.all(y[torch.from_numpy(none).to(cuda)] == 0)

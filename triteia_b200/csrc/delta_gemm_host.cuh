@@ -411,12 +411,9 @@ int sbmm_indexed_impl(const void* x, const void* qweights, const void* metas, co
 
   int r = TRB_OK;
   if (phases & 1) {
-    r = route_launch_src(src, num_tokens, num_deltas, kSmallTile, perm, nullptr, nullptr, nullptr, small.tile_delta,
-                         small.tile_start, small.tile_count, counters, nullptr, 0, nullptr, stream,
-                         use_big ? &cl : nullptr);
-    if (r != TRB_OK) return r;
-    r = gather_launch(x, perm, counters, x_sorted, y, num_tokens, prob_k, prob_m, mode == 0 ? 1 : 0, stream,
-                      ksplit ? counters + kKsplitCntOffset : nullptr, kKsplitItems);
+    r = route_gather_launch(src, num_tokens, num_deltas, kSmallTile, perm, small, counters, use_big ? &cl : nullptr, x,
+                            x_sorted, y, prob_k, prob_m, mode == 0 ? 1 : 0,
+                            ksplit ? counters + kKsplitCntOffset : nullptr, kKsplitItems, stream);
     if (r != TRB_OK) return r;
   }
   if (!(phases & 2)) return TRB_OK;

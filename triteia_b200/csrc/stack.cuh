@@ -133,13 +133,14 @@ extern "C" int trb_stack_pass(int n_linears, const void* const* q, const void* c
   cl.big = big;
   RouteSrc src{};
   src.indices = (const int*)ids;
-  int r = route_launch_src(src, rows, num_deltas, kSmallTile, perm, nullptr, nullptr, nullptr, small.tile_delta,
-                           small.tile_start, small.tile_count, counters, nullptr, 0, nullptr, stream, use_big ? &cl : nullptr);
+  // the first gather also clears the rows of y_last whose id selects no delta
+  int r = route_gather_launch(src, rows, num_deltas, kSmallTile, perm, small, counters, use_big ? &cl : nullptr, x_of_width[0],
+                              xs_of_width[0], y_last, width[0], n[n_linears - 1], 1, counters + kKsplitCntOffset,
+                              kKsplitItems, stream);
   if (r != TRB_OK) return r;
-  for (int w = 0; w < n_widths; ++w) {
-    // the first gather also clears the rows of y_last whose id selects no delta
-    r = gather_launch(x_of_width[w], perm, counters, xs_of_width[w], w == 0 ? y_last : nullptr, rows, width[w],
-                      n[n_linears - 1], w == 0 ? 1 : 0, stream, w == 0 ? counters + kKsplitCntOffset : nullptr, kKsplitItems);
+  for (int w = 1; w < n_widths; ++w) {
+    r = gather_launch(x_of_width[w], perm, counters, xs_of_width[w], nullptr, rows, width[w], n[n_linears - 1], 0, stream,
+                      nullptr, kKsplitItems);
     if (r != TRB_OK) return r;
   }
   for (int i = 0; i < n_linears; ++i) {
