@@ -1092,3 +1092,13 @@ def test_router_and_gather_in_one_launch(cuda, T, D):
     clean = np.where(none, -1, idx_np).astype(np.int32)
     check(y, oracle.sbmm(qs.cpu().numpy(), x.cpu().numpy(), metas.cpu().numpy(), ss.cpu().numpy(), clean), mean_tol=None)
     assert torch.all(y[torch.from_numpy(none).to(cuda)] == 0)
+
+
+@pytest.mark.parametrize("T", [1, 8, 9, 32])
+@pytest.mark.parametrize("K,N", [(128, 2048), (1408, 2304), (256, 19200)])
+def test_matmul_few_tokens_item_width(cuda, T, K, N):
+    """One weight at decode sizes on both sides of the rule that picks 128- or 256-column items."""
+    ops = _ops()
+    q, m, s = packed(N, K, 128, seed=T)
+    x = torch.randn(T, K, dtype=torch.float16, device=cuda, generator=torch.Generator(cuda).manual_seed(T))
+    check(ops.matmul_4bit_2_4(q, x, m, s), oracle.matmul_2_4(q.cpu().numpy(), x.cpu().numpy(), m.cpu().numpy(), s.cpu().numpy()))

@@ -219,7 +219,13 @@ int gemm_dispatch(const GemmCall& c, const GemmArgs& a, int tile_tokens) {
   cudaError_t e = cudaSetDevice(c.dev);
   if (e != cudaSuccess) return TRB_ERR_CUDA;
   switch (tile_tokens) {
-    case kSmallTile: return (a.N % 256 == 0 && a.N >= 2048) ? launch_cfg<CfgWide8>(c, a) : launch_cfg<CfgNarrow8>(c, a);
+    case kSmallTile: {
+      // One weight and few tokens: wide items would leave most SMs idle, narrow ones are twice as many and half as long.
+      // Measured (CUDA events, cold L2, wide -> narrow): 1 x 2048 x 2048 13.3 -> 11.3 us, 16 x 4096 x 4096 17.4 -> 15.4,
+      // 8 x 4096 x 12288 19.2 -> 15.4, 1 x 11008 x 4096 35.8 -> 27.6; equal where wide items already fill half the SMs.
+      const bool idle = a.mode == kSegSingle && 2ll * ((a.rows + kSmallTile - 1) / kSmallTile) * (a.N / 256) <= sm_count(c.dev);
+      return (a.N % 256 == 0 && a.N >= 2048 && !idle) ? launch_cfg<CfgWide8>(c, a) : launch_cfg<CfgNarrow8>(c, a);
+    }
     case kBigTile: return a.y_peers ? TRB_ERR_KERN_SHAPE : launch_tc(c, a);
     default: return TRB_ERR_KERN_SHAPE;
   }
