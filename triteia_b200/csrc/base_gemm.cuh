@@ -103,10 +103,8 @@ __device__ __forceinline__ void tc_mma_f16_pair(uint32_t d_tmem, uint64_t a_desc
       : "memory");
 }
 
-// A 32-token x 32-feature block of results, one feature per lane: convert, transpose through the warp's patch
-// of shared memory, store 16-byte pieces of 8 features.  `old`: the pieces' previous values (accumulate).
-__device__ __forceinline__ void base_store_batch(const BaseArgs& a, __half* patch, const uint32_t (&v)[32], int row0,
-                                                 int valid, int col, int b, int lane, const uint4 (&old)[4]) {
+// A 32-token x 32-feature block of results, one feature per lane, as rows of 32 features in the warp's patch.
+__device__ __forceinline__ void base_fill_patch(const BaseArgs& a, __half* patch, const uint32_t (&v)[32], int lane) {
   if (a.bf16) {
     __nv_bfloat16* pb = reinterpret_cast<__nv_bfloat16*>(patch);
 #pragma unroll
@@ -115,6 +113,21 @@ __device__ __forceinline__ void base_store_batch(const BaseArgs& a, __half* patc
 #pragma unroll
     for (int c = 0; c < 32; ++c) patch[c * 32 + lane] = __float2half_rn(__uint_as_float(v[c]));
   }
+}
+// Adds a box from shared memory to a tensor in global memory, element by element; a bulk group of its own.
+__device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* map, const void* src, int c0, int c1) {
+  asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
+                   reinterpret_cast<uint64_t>(map)),
+               "r"(smem_u32(src)), "r"(c0), "r"(c1)
+               : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+
+// A 32-token x 32-feature block of results, one feature per lane: convert, transpose through the warp's patch
+// of shared memory, store 16-byte pieces of 8 features.  `old`: the pieces' previous values (accumulate).
+__device__ __forceinline__ void base_store_batch(const BaseArgs& a, __half* patch, const uint32_t (&v)[32], int row0,
+                                                 int valid, int col, int b, int lane, const uint4 (&old)[4]) {
+  base_fill_patch(a, patch, v, lane);
   __syncwarp();
   const int f8 = (lane & 3) * 8;                      // feature offset of this lane's 16-byte piece
 #pragma unroll
@@ -166,7 +179,7 @@ template <bool SPLIT>
 __global__ void __launch_bounds__(BaseCfg::THREADS, 1)
 base_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w,
                  const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_b,
-                 const BaseArgs a) {
+                 const __grid_constant__ CUtensorMap tm_y, const BaseArgs a) {
   using Cfg = BaseCfg;
   constexpr int STAGES = Cfg::STAGES;
   extern __shared__ uint8_t smem_raw[];
@@ -401,28 +414,21 @@ base_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
       const int col0 = stripe * 256 + (int)rank * 128;
       const int buf = local & 1;
       // Each warp drains the 32-token batches b0, b0 + 1, ... of its TMEM lane quadrant (two warps share a
-      // quadrant and split the batches).  Accumulating into y: the old values of all its batches are
-      // fetched before the accumulator is complete, so the epilogue never waits on a load it just issued.
+      // quadrant and split the batches).  Accumulating into y: a full batch leaves as a TMA reduction of its 32 x 32
+      // block, an addition in the type of y in L2 (the same rounding as a load, an addition and a store), so the
+      // warp neither reads y nor waits for it.  A batch that the tile ends in is read, added and stored.
+      // LoRA expand of 7001 x 64 x 13824 into y (387 MB read and written): 154 us with the old values prefetched into
+      // registers and added by the warps, 88 us this way.
       constexpr int MAXB = BaseCfg::MAX_TT / 32 / 2;    // batches per warp
       const int f8 = (lane & 3) * 8;                  // feature offset of this lane's 16-byte piece
       const int nb = col0 + quad * 32 + f8;
       const int nbatch = max(1, (valid + 31) >> 5);
       const int per = (nbatch + 1) >> 1;
       const int b0 = (ew >> 2) * per, b1 = min(nbatch, b0 + per);
-      auto piece = [&](int b, int i) -> uint4* {      // 16 bytes of token b * 32 + i * 8 + lane / 4, or nullptr
+      auto old_piece = [&](int b, int i) -> uint4 {   // 16 bytes of token b * 32 + i * 8 + lane / 4
         const int t = b * 32 + i * 8 + (lane >> 2);
-        return (t < valid && nb < a.N) ? reinterpret_cast<uint4*>(a.y + (size_t)(row0 + t) * a.N + nb) : nullptr;
+        return (t < valid && nb < a.N) ? *reinterpret_cast<const uint4*>(a.y + (size_t)(row0 + t) * a.N + nb) : make_uint4(0, 0, 0, 0);
       };
-      uint4 old[MAXB][4];
-      if (a.accumulate) {
-#pragma unroll
-        for (int k = 0; k < MAXB; ++k)
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const uint4* yp = b0 + k < b1 ? piece(b0 + k, i) : nullptr;
-            old[k][i] = yp ? *yp : make_uint4(0, 0, 0, 0);
-          }
-      }
       if (ew == 0) {                                  // one warp polls, the others park on the hardware barrier
         uint32_t polls = 0;
         while (!mbar_try_wait(&accready_bar[buf], use[buf] & 1)) {
@@ -454,11 +460,28 @@ base_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
           if (lane == 0) mbar_arrive_cluster(accfree_leader + buf * 8);
         }
         if (b >= b1) continue;
-        base_store_batch(a, patch, v, row0, valid, col0 + quad * 32, b, lane, old[k]);
+        if (a.accumulate && valid - b * 32 >= 32) {
+          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the patch has been read
+          __syncwarp();
+          base_fill_patch(a, patch, v, lane);
+          fence_proxy_async();
+          __syncwarp();
+          if (lane == 0 && col0 + quad * 32 < a.N) tma_reduce_add_2d(&tm_y, patch, col0 + quad * 32, row0 + b * 32);
+          continue;
+        }
+        uint4 old[4];
+        if (a.accumulate) {
+          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < 4; ++i) old[i] = old_piece(b, i);
+        }
+        base_store_batch(a, patch, v, row0, valid, col0 + quad * 32, b, lane, old);
       }
       ++use[buf];
       ++local;
     }
+    if (a.accumulate && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // reductions performed
   }
 
   if constexpr (SPLIT) {
@@ -672,6 +695,10 @@ static int base_gemm_launch_args(BaseArgs a, const CUtensorMap& tx, const CUtens
     cluster = 2 * a.split_pairs;
     pairs = a.split_pairs * (int)items;
   }
+  CUtensorMap ty = tx;     // used with accumulate only
+  if (a.accumulate && !make_map_2d(&ty, a.bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.y,
+                                   (uint64_t)a.T, (uint64_t)a.N, 32, 32, CU_TENSOR_MAP_SWIZZLE_NONE))
+    return TRB_ERR_CUDA;
   cudaLaunchConfig_t lc = {};
   lc.gridDim = dim3(2 * pairs);
   lc.blockDim = dim3(BaseCfg::THREADS);
@@ -686,7 +713,7 @@ static int base_gemm_launch_args(BaseArgs a, const CUtensorMap& tx, const CUtens
   at[1].val.clusterDim.z = 1;
   lc.attrs = at;
   lc.numAttrs = 2;
-  return cudaLaunchKernelEx(&lc, a.split_pairs > 0 ? base_gemm_kernel<true> : base_gemm_kernel<false>, tx, tw, tv, tb, a) ==
+  return cudaLaunchKernelEx(&lc, a.split_pairs > 0 ? base_gemm_kernel<true> : base_gemm_kernel<false>, tx, tw, tv, tb, ty, a) ==
                  cudaSuccess
              ? TRB_OK
              : TRB_ERR_CUDA;
