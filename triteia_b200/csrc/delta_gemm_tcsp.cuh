@@ -27,14 +27,14 @@
 // epilogue of a small tile overlaps the next one's chunks), then 32 columns of weights and 4 of metadata
 // per stage.
 //
-// What bounds it: the 128 B/clk shared-memory pipe of an SM.  Per 64 K a 256-token tile needs 128
-// wavefronts for the activations landing, 128 for the tensor core reading them, 25 for the packed
-// weights and about 50 for their decode, against 247 cycles of the instruction.  Weights in shared memory
-// would add 64 for the decode's stores and 64 for the tensor core, and a proxy fence on the decode
-// warps' chain.
+// What bounds it (in-kernel cycle counters): a loop of latencies over the five stages, load about 1200 to 1500
+// cycles, decode 700, MMA and hand-back 500, that is 520 to 650 cycles per 128 K against 494 of the instruction at
+// 256 tokens; and for 256-token tiles the drain of the accumulator, about 4000 cycles an item.  The shared-memory
+// pipe would be next: 512 wavefronts of activations landing and read, 50 of packed weights, about 100 of decode;
+// weights in shared memory would add 256 and a proxy fence on the decode warps' chain.
 // Measured, whole calls (before: weights through shared memory, 64-K stages, every tile as 256 tokens, one
-// accumulator): 8192 tokens in 16 segments, 5120 -> 13824: 857 -> 721 us; 1531 tokens, one weight, 4096 -> 11008:
-// 109 -> 91 us; 700 tokens over 13 deltas (54 each), 4096 -> 12288: 229 -> 127 us.
+// accumulator): 8192 tokens in 16 segments, 5120 -> 13824: 858 -> 705 us; 1531 tokens, one weight, 4096 -> 11008:
+// 109 -> 89 us; 700 tokens over 13 deltas (54 each), 4096 -> 12288: 228 -> 116 us.
 // Every wait is bounded; both CTAs of a pair meet at a cluster barrier before either leaves.
 #pragma once
 
