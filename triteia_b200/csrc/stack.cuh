@@ -1,8 +1,9 @@
 // Per-row fp32 checksum of an fp16 matrix: sums[r] (+)= sum over n of y[r, n].
 // The linear-stack scenario (many independent indexed delta matmuls over the same routed tokens)
 // reduces every linear's output to one number per token, so that the result a token owner gets back
-// covers all of them without shipping every output row.  One warp per row, 16-byte loads, fp32 adds
-// in a fixed order (lane-strided partial sums, then a butterfly), so results are run-to-run identical.
+// covers all of them without shipping every output row.  One CTA per row, 16-byte loads, fp32 adds
+// in a fixed order (thread-strided partial sums, a butterfly, the warps in turn), so results are run-to-run
+// identical.  Bound by reading y, mostly from L2: at 512 rows of 22016 a warp per row kept 64 CTAs busy, 17.9 us.
 // The reference has no counterpart (its benchmarks compare full outputs, one linear at a time).
 #pragma once
 
@@ -10,17 +11,19 @@
 
 namespace trb {
 
-__global__ void row_checksum_kernel(const uint4* __restrict__ y, float* __restrict__ sums, int rows, int n_vec,
-                                    int accumulate, const int* __restrict__ row_map,
-                                    const int* __restrict__ first_row) {
+constexpr int kChecksumThreads = 256;
+
+__global__ void __launch_bounds__(kChecksumThreads)
+row_checksum_kernel(const uint4* __restrict__ y, float* __restrict__ sums, int n_vec, int rows, int accumulate,
+                    const int* __restrict__ row_map, const int* __restrict__ first_row) {
+  __shared__ float part[kChecksumThreads / 32];
   pdl_wait();
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (warp >= rows) return;
-  if (first_row != nullptr && warp < *first_row) return;   // sorted order: rows without a delta come first and hold nothing
-  const uint4* row = y + (size_t)warp * n_vec;
+  const int r = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (first_row != nullptr && r < *first_row) return;   // sorted order: rows without a delta come first and hold nothing
+  const uint4* row = y + (size_t)r * n_vec;
   float acc = 0.f;
-  for (int i = lane; i < n_vec; i += 32) {
+#pragma unroll 4
+  for (int i = threadIdx.x; i < n_vec; i += kChecksumThreads) {
     const uint4 v = row[i];
     const __half2* h = reinterpret_cast<const __half2*>(&v);
 #pragma unroll
@@ -32,9 +35,14 @@ __global__ void row_checksum_kernel(const uint4* __restrict__ y, float* __restri
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if (lane == 0) {
-    const int out = row_map ? row_map[warp] : warp;      // row r of y is row row_map[r] of the caller's order
-    if (out >= 0 && out < rows) sums[out] = accumulate ? sums[out] + acc : acc;
+  if (lane == 0) part[warp] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float sum = 0.f;
+#pragma unroll
+    for (int w = 0; w < kChecksumThreads / 32; ++w) sum += part[w];
+    const int out = row_map ? row_map[r] : r;      // row r of y is row row_map[r] of the caller's order
+    if (out >= 0 && out < rows) sums[out] = accumulate ? sums[out] + sum : sum;
   }
 }
 
@@ -44,15 +52,15 @@ namespace trb {
 static int row_checksum_launch(const void* y, void* sums, int rows, int prob_m, int accumulate, const int* row_map,
                                const int* first_row, cudaStream_t stream) {
   cudaLaunchConfig_t lc = {};
-  lc.gridDim = dim3((rows + 7) / 8);
-  lc.blockDim = dim3(256);
+  lc.gridDim = dim3(rows);
+  lc.blockDim = dim3(kChecksumThreads);
   lc.stream = stream;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // the kernel waits before it reads y
   at[0].val.programmaticStreamSerializationAllowed = 1;
   lc.attrs = at;
   lc.numAttrs = 1;
-  return cudaLaunchKernelEx(&lc, row_checksum_kernel, (const uint4*)y, (float*)sums, rows, prob_m / 8, accumulate,
+  return cudaLaunchKernelEx(&lc, row_checksum_kernel, (const uint4*)y, (float*)sums, prob_m / 8, rows, accumulate,
                             row_map, first_row) == cudaSuccess
              ? TRB_OK
              : TRB_ERR_CUDA;
