@@ -90,13 +90,19 @@ def base_indexed(xs, base_weight, qweights, metas, ss, indices, weights_A=None, 
     adapters M = 0.  fp16; weights_A [M, K, r], weights_B [M, r, N] contiguous."""
     T, K = xs.shape
     D, G, N = ss.shape
+    M, rank = (0, 0) if weights_A is None else (weights_A.shape[0], weights_A.shape[2])
+    # The native call takes N from the deltas and K from xs: it would read past a smaller weight.
+    if tuple(base_weight.shape) != (N, K):
+        raise RuntimeError(f"base weight of shape {tuple(base_weight.shape)}: the deltas and inputs need ({N}, {K})")
+    if M and (tuple(weights_A.shape) != (M, K, rank) or tuple(weights_B.shape) != (M, rank, N)):
+        raise RuntimeError(f"adapters of shapes {tuple(weights_A.shape)} and {tuple(weights_B.shape)}: "
+                           f"the deltas and inputs need ({M}, {K}, {rank}) and ({M}, {rank}, {N})")
     if base_weight.dtype != xs.dtype:
         base_weight = base_weight.to(xs.dtype)
     if not base_weight.is_contiguous():
         base_weight = base_weight.contiguous()
     if indices.dtype != torch.int32:
         indices = indices.to(torch.int32)
-    M, rank = (0, 0) if weights_A is None else (weights_A.shape[0], weights_A.shape[2])
     y = torch.empty(T, N, dtype=xs.dtype, device=xs.device)
     v = torch.empty(T, M * rank, dtype=xs.dtype, device=xs.device) if M else None
     buf = scratch(xs.device, lib.trb_sbmm_indexed_scratch_bytes(T, K, D))
