@@ -1102,3 +1102,25 @@ def test_matmul_few_tokens_item_width(cuda, T, K, N):
     q, m, s = packed(N, K, 128, seed=T)
     x = torch.randn(T, K, dtype=torch.float16, device=cuda, generator=torch.Generator(cuda).manual_seed(T))
     check(ops.matmul_4bit_2_4(q, x, m, s), oracle.matmul_2_4(q.cpu().numpy(), x.cpu().numpy(), m.cpu().numpy(), s.cpu().numpy()))
+
+
+@pytest.mark.parametrize("groupsize", [-1, 128])
+def test_sbmm_long_segments_repeat_bit_for_bit(cuda, groupsize):
+    """Many passes over a batch whose tiles mix the tcgen05 kernel's three widths: several items per CTA pair, more
+    chunks than stages, weight tiles from HBM (L2 is overwritten every few passes, so that loads land out of order).
+    Every pass gives the same bits; a stage or tensor-memory column reused too early shows as a pass that differs."""
+    ops = _ops()
+    K, N, D = 2048, 4096, 9
+    qs, metas, ss = ops.random_packed_deltas(D, K, N, groupsize=groupsize, device=cuda, seed=6)
+    counts = [33, 64, 65, 128, 129, 256, 300, 54, 40]
+    idx = torch.from_numpy(np.repeat(np.arange(D), counts).astype(np.int32)).to(cuda)
+    x = torch.randn(len(idx), K, dtype=torch.float16, device=cuda, generator=torch.Generator(cuda).manual_seed(8))
+    flush = torch.empty(1 << 26, dtype=torch.int32, device=cuda)
+    first = ops.sbmm_4bit_2_4_native(qs, x, metas, ss, idx)
+    differ = torch.zeros((), dtype=torch.int64, device=cuda)
+    for i in range(600):
+        if i % 4 == 0:
+            flush.zero_()
+        differ += (ops.sbmm_4bit_2_4_native(qs, x, metas, ss, idx) != first).any()
+    assert int(differ) == 0
+    assert _lib().device_status(0) == 0

@@ -407,6 +407,7 @@ delta_gemm_tcsp_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_c
       for (int kc = 0; kc < k_chunks; ++kc) {
         if (turn == team) {
           mbar_wait(&full_bar[fb], phase, dead);
+          tc_fence_after();      // the stage's columns were read by MMAs: retired before TMA filled the stage again
           const uint32_t sb = smem_base + st * Cfg::STAGE_BYTES;
           uint32_t e[Cfg::SLABS];
 #pragma unroll
