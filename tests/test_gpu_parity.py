@@ -1124,3 +1124,20 @@ def test_sbmm_long_segments_repeat_bit_for_bit(cuda, groupsize):
         differ += (ops.sbmm_4bit_2_4_native(qs, x, metas, ss, idx) != first).any()
     assert int(differ) == 0
     assert _lib().device_status(0) == 0
+
+
+@pytest.mark.parametrize("groupsize", [-1, 128])
+def test_sbmm_short_segments_repeat_bit_for_bit(cuda, groupsize):
+    """Many passes over a decode batch (8-token tiles, every stage of the ring used several times, weights from HBM):
+    every pass gives the same bits; a stage refilled before its words were read shows as a pass that differs."""
+    ops = _ops()
+    K, N, D, T = 2048, 4096, 64, 100
+    qs, metas, ss = ops.random_packed_deltas(D, K, N, groupsize=groupsize, device=cuda, seed=6)
+    idx = torch.from_numpy(np.random.default_rng(5).integers(-1, D, T).astype(np.int32)).to(cuda)
+    x = torch.randn(T, K, dtype=torch.float16, device=cuda, generator=torch.Generator(cuda).manual_seed(8))
+    first = ops.sbmm_4bit_2_4_native(qs, x, metas, ss, idx)
+    differ = torch.zeros((), dtype=torch.int64, device=cuda)
+    for _ in range(2000):
+        differ += (ops.sbmm_4bit_2_4_native(qs, x, metas, ss, idx) != first).any()
+    assert int(differ) == 0
+    assert _lib().device_status(0) == 0
