@@ -1141,3 +1141,61 @@ def test_sbmm_short_segments_repeat_bit_for_bit(cuda, groupsize):
         differ += (ops.sbmm_4bit_2_4_native(qs, x, metas, ss, idx) != first).any()
     assert int(differ) == 0
     assert _lib().device_status(0) == 0
+
+
+UNIT = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}     # half the spacing of the type, relative
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("accumulate", [True, False])
+@pytest.mark.parametrize("N", [200, 504, 1000, 2600])
+@pytest.mark.parametrize("K", [24, 200])
+def test_sgmv_stacked_token_tiles(cuda, K, N, accumulate, dtype):
+    """The segmented form with token tiles of 32 (N = 200), 64, 128 and 256 (N = 2600): segments that end inside a tile, at its
+    edge and one past it, at odd first rows, one empty, and an N that ends inside a 32-column block, written and added.
+    Element by element: the product is rounded once to the type, the sum once more; the rest is fp32 summation.
+    Rows outside the segments keep their bits."""
+    from triteia_b200.ops.matmul.lora import sgmv_stacked
+    lens, lead, trail = [1, 31, 33, 0, 255, 257, 500], 3, 5
+    seg = np.cumsum([lead] + lens)
+    T = int(seg[-1]) + trail
+    g = torch.Generator(cuda).manual_seed(N + K)
+    x = torch.randn(T, K, device=cuda, generator=g).to(dtype)
+    w = torch.randn(len(lens), K, N, device=cuda, generator=g).to(dtype)
+    y0 = (torch.randn(T, N, device=cuda, generator=g) * K ** 0.5).to(dtype)
+    y = sgmv_stacked(y0.clone(), x, w, torch.from_numpy(seg.astype(np.int32)).to(cuda), accumulate=accumulate)
+    prod, mass = torch.zeros(T, N, device=cuda, dtype=torch.float64), torch.zeros(T, N, device=cuda, dtype=torch.float64)
+    for i in range(len(lens)):
+        r = slice(int(seg[i]), int(seg[i + 1]))
+        prod[r] = x[r].double() @ w[i].double()
+        mass[r] = x[r].double().abs() @ w[i].double().abs()
+    ref = prod + y0.double() if accumulate else prod
+    bound = 1.01 * UNIT[dtype] * (prod.abs() + (ref.abs() if accumulate else 0)) + K * 2.0 ** -23 * mass
+    inside = slice(lead, T - trail)
+    assert ((y.double() - ref).abs() <= bound)[inside].all()
+    assert torch.equal(y[:lead], y0[:lead]) and torch.equal(y[T - trail:], y0[T - trail:])
+    assert _lib().device_status(0) == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_accumulating_product_special_values(cuda, dtype):
+    """What is added to y, by TMA reductions (full blocks of 32 tokens) and by the warps (the last 13), for
+    subnormal, infinite, NaN and overflowing sums: the bits of an addition in fp32 rounded once to the type."""
+    from triteia_b200.ops.matmul.lora import sgmv_stacked
+    info = torch.finfo(dtype)
+    vals = torch.tensor([0.0, info.smallest_normal, info.smallest_normal / 2, info.tiny / 8, -info.tiny / 4, 3 * info.tiny / 8, 1.0,
+                         -1.0, 1.0 + info.eps, info.max, -info.max, info.max / 2, 1.5, 2.0 ** -9, -2.0 ** -9, 7.25],
+                        device=cuda, dtype=torch.float64).to(dtype)
+    old = torch.cat([vals, torch.tensor([float("inf"), -float("inf"), float("nan"), -0.0], device=cuda, dtype=dtype)])
+    T, K, N = 45, 64, vals.numel() * old.numel()
+    w = torch.zeros(1, K, N, device=cuda, dtype=dtype)
+    w[0, :] = vals.repeat(old.numel())                    # every token picks one row of w: the product is exact
+    x = torch.zeros(T, K, device=cuda, dtype=dtype)
+    x[torch.arange(T), torch.arange(T) % K] = 1.0
+    y0 = old.repeat_interleave(vals.numel()).repeat(T, 1)
+    y = sgmv_stacked(y0.clone(), x, w, torch.tensor([0, T], device=cuda, dtype=torch.int32), accumulate=True)
+    ref = (y0.float() + w[0, 0].float()).to(dtype)
+    nan = torch.isnan(ref)
+    assert torch.equal(torch.isnan(y), nan)
+    assert torch.equal(y[~nan], ref[~nan])
+    assert _lib().device_status(0) == 0

@@ -124,7 +124,8 @@ __device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* map, const 
 }
 
 // A 32-token x 32-feature block of results, one feature per lane: convert, transpose through the warp's patch
-// of shared memory, store 16-byte pieces of 8 features.  `old`: the pieces' previous values (accumulate).
+// of shared memory, store 16-byte pieces of 8 features.  `old`: the pieces' previous values (ADD).
+template <bool ADD>
 __device__ __forceinline__ void base_store_batch(const BaseArgs& a, __half* patch, const uint32_t (&v)[32], int row0,
                                                  int valid, int col, int b, int lane, const uint4 (&old)[4]) {
   base_fill_patch(a, patch, v, lane);
@@ -136,7 +137,7 @@ __device__ __forceinline__ void base_store_batch(const BaseArgs& a, __half* patc
     const int t = b * 32 + c;
     if (t < valid && col + f8 < a.N) {
       uint4 o = *reinterpret_cast<const uint4*>(patch + c * 32 + f8);
-      if (a.accumulate) {
+      if constexpr (ADD) {
         if (a.bf16) {
           __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
           const __nv_bfloat162* ph = reinterpret_cast<const __nv_bfloat162*>(&old[i]);
@@ -175,7 +176,9 @@ struct BaseUnit {
 // every accumulator of the cluster is complete, each pair sends the token batches that another pair finishes
 // as fp32 into that pair's shared memory (the stage ring, idle by then) and adds what it receives for its own
 // batches in the order of the ranges.  Everything stays inside the cluster: no workspace, no counters.
-template <bool SPLIT>
+// ADD: the result is added to y.  A form of its own: with both epilogues in one kernel the plain one was slower
+// (7001 x 64 -> 13824 into a fresh y 89 -> 105 us, 8192 x 64 -> 5120 41 -> 49, 300 x 512 x 512 8.4 -> 9.9).
+template <bool SPLIT, bool ADD>
 __global__ void __launch_bounds__(BaseCfg::THREADS, 1)
 base_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w,
                  const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_b,
@@ -425,10 +428,6 @@ base_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
       const int nbatch = max(1, (valid + 31) >> 5);
       const int per = (nbatch + 1) >> 1;
       const int b0 = (ew >> 2) * per, b1 = min(nbatch, b0 + per);
-      auto old_piece = [&](int b, int i) -> uint4 {   // 16 bytes of token b * 32 + i * 8 + lane / 4
-        const int t = b * 32 + i * 8 + (lane >> 2);
-        return (t < valid && nb < a.N) ? *reinterpret_cast<const uint4*>(a.y + (size_t)(row0 + t) * a.N + nb) : make_uint4(0, 0, 0, 0);
-      };
       if (ew == 0) {                                  // one warp polls, the others park on the hardware barrier
         uint32_t polls = 0;
         while (!mbar_try_wait(&accready_bar[buf], use[buf] & 1)) {
@@ -460,28 +459,33 @@ base_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
           if (lane == 0) mbar_arrive_cluster(accfree_leader + buf * 8);
         }
         if (b >= b1) continue;
-        if (a.accumulate && valid - b * 32 >= 32) {
+        if constexpr (ADD) {
           if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the patch has been read
           __syncwarp();
-          base_fill_patch(a, patch, v, lane);
-          fence_proxy_async();
-          __syncwarp();
-          if (lane == 0 && col0 + quad * 32 < a.N) tma_reduce_add_2d(&tm_y, patch, col0 + quad * 32, row0 + b * 32);
-          continue;
+          if (valid - b * 32 >= 32) {
+            base_fill_patch(a, patch, v, lane);
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0 && col0 + quad * 32 < a.N) tma_reduce_add_2d(&tm_y, patch, col0 + quad * 32, row0 + b * 32);
+            continue;
+          }
         }
         uint4 old[4];
-        if (a.accumulate) {
-          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-          __syncwarp();
+        if constexpr (ADD) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) old[i] = old_piece(b, i);
+          for (int i = 0; i < 4; ++i) {
+            const int t = b * 32 + i * 8 + (lane >> 2);
+            old[i] = (t < valid && nb < a.N) ? *reinterpret_cast<const uint4*>(a.y + (size_t)(row0 + t) * a.N + nb) : make_uint4(0, 0, 0, 0);
+          }
         }
-        base_store_batch(a, patch, v, row0, valid, col0 + quad * 32, b, lane, old);
+        base_store_batch<ADD>(a, patch, v, row0, valid, col0 + quad * 32, b, lane, old);
       }
       ++use[buf];
       ++local;
     }
-    if (a.accumulate && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // reductions performed
+    if constexpr (ADD) {
+      if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // reductions performed
+    }
   }
 
   if constexpr (SPLIT) {
@@ -529,7 +533,7 @@ base_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
         for (int i = 0; i < 4; ++i) {
           const int t = b * 32 + i * 8 + (lane >> 2), col = col0 + (lane & 3) * 8;
           old[i] = make_uint4(0, 0, 0, 0);
-          if (a.accumulate && t < valid && col < a.N) old[i] = *reinterpret_cast<const uint4*>(a.y + (size_t)(row0 + t) * a.N + col);
+          if (ADD && t < valid && col < a.N) old[i] = *reinterpret_cast<const uint4*>(a.y + (size_t)(row0 + t) * a.N + col);
         }
         uint32_t own[32], v[32];
         tc_ld32(taddr + b * 32, own);
@@ -552,7 +556,7 @@ base_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
             }
           }
         }
-        base_store_batch(a, patch, v, row0, valid, col0, b, lane, old);
+        base_store_batch<ADD>(a, patch, v, row0, valid, col0, b, lane, old);
       }
     }
   }
@@ -660,7 +664,7 @@ static int max_split_clusters(int dev, int pairs) {
     lc.attrs = at;
     lc.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, base_gemm_kernel<true>, &lc) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&n, base_gemm_kernel<true, false>, &lc) != cudaSuccess) {
       cudaGetLastError();
       n = 0;
     }
@@ -683,9 +687,12 @@ static int choose_split(int dev, long long items, int k_chunks) {
 
 static int base_gemm_launch_args(BaseArgs a, const CUtensorMap& tx, const CUtensorMap& tw, const CUtensorMap& tv,
                                  const CUtensorMap& tb, long long items, int dev, cudaStream_t stream) {
-  static std::atomic<bool> attr_set[64], attr_set_split[64];
-  if (!ensure_smem_attr(base_gemm_kernel<false>, dev, BaseCfg::SMEM_ALLOC, attr_set)) return TRB_ERR_CUDA;
-  if (!ensure_smem_attr(base_gemm_kernel<true>, dev, BaseCfg::SMEM_ALLOC, attr_set_split)) return TRB_ERR_CUDA;
+  static std::atomic<bool> attr_set[4][64];
+  if (!ensure_smem_attr(base_gemm_kernel<false, false>, dev, BaseCfg::SMEM_ALLOC, attr_set[0]) ||
+      !ensure_smem_attr(base_gemm_kernel<false, true>, dev, BaseCfg::SMEM_ALLOC, attr_set[1]) ||
+      !ensure_smem_attr(base_gemm_kernel<true, false>, dev, BaseCfg::SMEM_ALLOC, attr_set[2]) ||
+      !ensure_smem_attr(base_gemm_kernel<true, true>, dev, BaseCfg::SMEM_ALLOC, attr_set[3]))
+    return TRB_ERR_CUDA;
   int pairs = sm_count(dev) / 2;
   if (pairs < 1) pairs = 1;
   if (items < pairs) pairs = (int)(items > 0 ? items : 1);
@@ -713,10 +720,9 @@ static int base_gemm_launch_args(BaseArgs a, const CUtensorMap& tx, const CUtens
   at[1].val.clusterDim.z = 1;
   lc.attrs = at;
   lc.numAttrs = 2;
-  return cudaLaunchKernelEx(&lc, a.split_pairs > 0 ? base_gemm_kernel<true> : base_gemm_kernel<false>, tx, tw, tv, tb, ty, a) ==
-                 cudaSuccess
-             ? TRB_OK
-             : TRB_ERR_CUDA;
+  auto kernel = a.split_pairs > 0 ? (a.accumulate ? base_gemm_kernel<true, true> : base_gemm_kernel<true, false>)
+                                  : (a.accumulate ? base_gemm_kernel<false, true> : base_gemm_kernel<false, false>);
+  return cudaLaunchKernelEx(&lc, kernel, tx, tw, tv, tb, ty, a) == cudaSuccess ? TRB_OK : TRB_ERR_CUDA;
 }
 
 static int token_tile_for(int rows) { return rows <= 32 ? 32 : rows <= 64 ? 64 : rows <= 128 ? 128 : 256; }
