@@ -857,6 +857,30 @@ def test_base_gemm_split_and_order(cuda, T, K, N, M, dtype):
     assert _lib().device_status(0) == 0
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("T,K,N,M", [(1, 1280, 264, 0), (1, 1344, 264, 0), (100, 1600, 2048, 3), (300, 1984, 4096, 0),
+                                     (300, 2112, 4096, 0)])
+def test_base_gemm_on_both_sides_of_the_split_rule(cuda, T, K, N, M, dtype):
+    """20 chunks of K whole and 21 on four CTA pairs, 26 on four with LoRA chunks in the last range, 31 whole and 33 on two
+    pairs.  Element by element against 64 bits: one rounding to the type, a second one when added to y, fp32 sums."""
+    from triteia_b200.ops.matmul._base import base_gemm
+    g = torch.Generator(cuda).manual_seed(T + K + N)
+    x = torch.randn(T, K, device=cuda, generator=g).to(dtype)
+    w = (torch.randn(N, K, device=cuda, generator=g) * 0.05).to(dtype)
+    v = torch.randn(T, 16 * M, device=cuda, generator=g).to(dtype) if M else None
+    b = (torch.randn(16 * M, N, device=cuda, generator=g) * 0.2).to(dtype) if M else None
+    ref, mass = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    if M:
+        ref, mass = ref + v.double() @ b.double(), mass + v.double().abs() @ b.double().abs()
+    y = base_gemm(x, w, lora_v=v, lora_b=b)
+    unit, sums = 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8, (K + 16 * M) * 2.0 ** -23 * mass
+    assert ((y.double() - ref).abs() <= 1.01 * unit * ref.abs() + sums).all()
+    y2 = base_gemm(x, w, lora_v=v, lora_b=b, out=y.clone(), accumulate=True)
+    total = ref + y.double()
+    assert ((y2.double() - total).abs() <= 1.01 * unit * (ref.abs() + total.abs()) + sums).all()
+    assert _lib().device_status(0) == 0
+
+
 @pytest.mark.parametrize("groupsize", [-1, 128])
 @pytest.mark.parametrize("K,N", [(128, 384), (896, 512)])
 @pytest.mark.parametrize("counts", [(33, 64, 65), (128, 129, 40), (256, 257, 1), (385, 63, 192)])

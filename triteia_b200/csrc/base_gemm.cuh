@@ -680,13 +680,18 @@ static int max_split_clusters(int dev, int pairs) {
 }
 
 // CTA pairs that share an item of a product with `items` items of `k_chunks` chunks: four or two, when all clusters
-// run in one round and a pair keeps at least four chunks; otherwise 0.  The exchange costs about 4 us, a chunk 0.27.
-// Measured (CUDA events, cold L2; whole items -> split): 100 x 2048 x 2048 20.5 -> 18.4 us, 16 x 4096 x 4096
-// 28.7 -> 24.6, 64 x 4096 x 5120 29.5 -> 25.3, 1 x 11008 x 4096 60.4 -> 39.8.  Three pairs on two items, which
-// would use the pairs that 43 items leave idle, lost: 256 x 4096 x 11008 34.8 -> 38.9, 256 x 2048 x 9216 23.4 -> 31.5.
+// run in one round and a pair is spared at least kSplitSaved chunks; otherwise 0.  The exchange costs about 2.4 us, a
+// chunk 0.15 (narrow token tiles) to 0.27.
+// Measured (device time of a call behind an L2 flush; whole items -> split): 100 x 2048 x 2048 12.6 -> 10.8 us,
+// 32 x 4096 x 4096 19.8 -> 15.6, 512 x 4096 x 4096 26.7 -> 22.5, 64 x 3072 x 3072 16.5 -> 12.4; about the line
+// 64 x 1536 x 1536 10.3 -> 10.0, 512 x 2048 x 4096 (two pairs) 16.7 -> 16.5; below it, where items stay whole,
+// 64 x 512 x 512 6.1 -> 6.9, 100 x 768 x 3072 8.2 -> 9.5, 64 x 1024 x 4096 8.5 -> 9.3, 512 x 1024 x 4096 12.3 -> 13.3.
+// Three pairs on two items, which would use the pairs that 43 items leave idle, lost: 256 x 4096 x 11008
+// 34.8 -> 38.9, 256 x 2048 x 9216 23.4 -> 31.5.
+constexpr int kSplitSaved = 16;
 static int choose_split(int dev, long long items, int k_chunks) {
   for (int p = 4; p >= 2; p -= 2)
-    if (k_chunks >= 4 * p && items <= max_split_clusters(dev, p)) return p;
+    if (k_chunks - k_chunks / p >= kSplitSaved && items <= max_split_clusters(dev, p)) return p;
   return 0;
 }
 
