@@ -299,8 +299,10 @@ base_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
         prefetch_tmap(&tm_v);
         prefetch_tmap(&tm_b);
       }
-      // A weight tile that one token tile reads is read once; otherwise the pairs of a round share it.
-      const uint64_t pol_w = n_tiles > 1 ? policy_evict_normal() : policy_evict_first();
+      // The token tiles of a round share a weight tile, and with up to three token tiles one round reads it: evict-first
+      // (300 x 4096 x 11008 51.3 -> 46.8 us, 512: 51.7 -> 47.5, 700: 51.4 -> 49.2); more token tiles come back to it
+      // (1024: 78.9 / 78.2, 2048: 139.6 kept, 149.3 evict-first).
+      const uint64_t pol_w = n_tiles > 3 ? policy_evict_normal() : policy_evict_first();
       const uint64_t pol_x = policy_evict_last();
       const uint32_t stage_tx = Cfg::A_BYTES + half_tt * Cfg::KC * 2;
       int st = 0;
