@@ -625,6 +625,19 @@ def test_row_checksum(cuda, rows, n):
     assert _lib.lib.trb_row_checksum(_lib.ptr(y), _lib.ptr(sums), rows, n + 1, 0, _lib.dev_of(y), _lib.stream_of(y)) != 0
 
 
+@pytest.mark.parametrize("rows,n", [(5, 2048), (9, 2056), (342, 2056), (343, 2056), (4099, 128)])
+def test_row_checksum_warp_or_block_per_row(cuda, rows, n):
+    """Both sides of the rule that gives a row to a warp or to a CTA, rows that fill no whole CTA of warps: against 64 bits,
+    within the rounding of n fp32 additions."""
+    from triteia_b200 import _lib
+    y = torch.randn(rows, n, device=cuda, generator=torch.Generator(cuda).manual_seed(n)).half()
+    sums = torch.full((rows + 8,), 5.0, device=cuda)
+    _lib.check(_lib.lib.trb_row_checksum(_lib.ptr(y), _lib.ptr(sums), rows, n, 1, 0, _lib.stream_of(y)), "row_checksum")
+    bound = (n / 32 + 16) * 2.0 ** -24 * (y.double().abs().sum(1) + 5)
+    assert ((sums[:rows].double() - y.double().sum(1) - 5).abs() <= bound).all()
+    assert (sums[rows:] == 5).all()
+
+
 @pytest.mark.parametrize("segs,tokens", [(3, 5), (20, 40), (40, 100)])
 def test_segment_list_tail_k_split(cuda, segs, tokens):
     """trb_sbmm_2_4_ksplit: few work items (every one is a split tail item), a mix, and a launch whose

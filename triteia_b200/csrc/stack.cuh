@@ -1,9 +1,9 @@
 // Per-row fp32 checksum of an fp16 matrix: sums[r] (+)= sum over n of y[r, n].
 // The linear-stack scenario (many independent indexed delta matmuls over the same routed tokens)
 // reduces every linear's output to one number per token, so that the result a token owner gets back
-// covers all of them without shipping every output row.  One CTA per row, 16-byte loads, fp32 adds
+// covers all of them without shipping every output row.  One CTA or one warp per row, 16-byte loads, fp32 adds
 // in a fixed order (thread-strided partial sums, a butterfly, the warps in turn), so results are run-to-run
-// identical.  Bound by reading y, mostly from L2: at 512 rows of 22016 a warp per row kept 64 CTAs busy, 17.9 us.
+// identical.  Bound by reading y, mostly from L2.
 // The reference has no counterpart (its benchmarks compare full outputs, one linear at a time).
 #pragma once
 
@@ -11,19 +11,24 @@
 
 namespace trb {
 
-constexpr int kChecksumThreads = 256;
+constexpr int kChecksumThreads = 256, kChecksumWarps = kChecksumThreads / 32;
 
+// WPR warps share a row: a CTA takes kChecksumWarps / WPR rows.
+template <int WPR>
 __global__ void __launch_bounds__(kChecksumThreads)
 row_checksum_kernel(const uint4* __restrict__ y, float* __restrict__ sums, int n_vec, int rows, int accumulate,
                     const int* __restrict__ row_map, const int* __restrict__ first_row) {
-  __shared__ float part[kChecksumThreads / 32];
+  static_assert(WPR == 1 || WPR == kChecksumWarps, "a warp or a CTA per row");
+  __shared__ float part[kChecksumWarps];
   pdl_wait();
-  const int r = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int r = WPR == 1 ? blockIdx.x * kChecksumWarps + warp : blockIdx.x;
+  if (r >= rows) return;
   if (first_row != nullptr && r < *first_row) return;   // sorted order: rows without a delta come first and hold nothing
   const uint4* row = y + (size_t)r * n_vec;
   float acc = 0.f;
 #pragma unroll 4
-  for (int i = threadIdx.x; i < n_vec; i += kChecksumThreads) {
+  for (int i = WPR == 1 ? lane : threadIdx.x; i < n_vec; i += WPR * 32) {
     const uint4 v = row[i];
     const __half2* h = reinterpret_cast<const __half2*>(&v);
 #pragma unroll
@@ -35,14 +40,16 @@ row_checksum_kernel(const uint4* __restrict__ y, float* __restrict__ sums, int n
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if (lane == 0) part[warp] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float sum = 0.f;
+  if constexpr (WPR > 1) {
+    if (lane == 0) part[warp] = acc;
+    __syncthreads();
+    acc = 0.f;
 #pragma unroll
-    for (int w = 0; w < kChecksumThreads / 32; ++w) sum += part[w];
+    for (int w = 0; w < WPR; ++w) acc += part[w];
+  }
+  if (lane == 0 && (WPR == 1 || warp == 0)) {
     const int out = row_map ? row_map[r] : r;      // row r of y is row row_map[r] of the caller's order
-    if (out >= 0 && out < rows) sums[out] = accumulate ? sums[out] + sum : sum;
+    if (out >= 0 && out < rows) sums[out] = accumulate ? sums[out] + acc : acc;
   }
 }
 
@@ -52,7 +59,12 @@ namespace trb {
 static int row_checksum_launch(const void* y, void* sums, int rows, int prob_m, int accumulate, const int* row_map,
                                const int* first_row, cudaStream_t stream) {
   cudaLaunchConfig_t lc = {};
-  lc.gridDim = dim3(rows);
+  // A CTA per row where warps would leave the SMs idle (few rows) and the row is long enough for 256 threads.
+  // Measured (device time behind an L2 flush, warp per row / CTA per row): 512 x 22016 16.1 / 8.2 us, 128 x 4096
+  // 3.7 / 2.1, 512 x 4096 4.1 / 4.1; 1200 x 4096 4.6 / 6.1, 4096 x 4096 8.3 / 11.8, 512 x 2048 2.3 / 3.6,
+  // 8192 x 128 2.0 / 10.5, 4096 x 22016 37.1 / 39.0.
+  const bool warp_rows = prob_m <= 2048 || 6ll * rows >= prob_m;
+  lc.gridDim = dim3(warp_rows ? (rows + kChecksumWarps - 1) / kChecksumWarps : rows);
   lc.blockDim = dim3(kChecksumThreads);
   lc.stream = stream;
   cudaLaunchAttribute at[1];
@@ -60,7 +72,7 @@ static int row_checksum_launch(const void* y, void* sums, int rows, int prob_m, 
   at[0].val.programmaticStreamSerializationAllowed = 1;
   lc.attrs = at;
   lc.numAttrs = 1;
-  return cudaLaunchKernelEx(&lc, row_checksum_kernel, (const uint4*)y, (float*)sums, prob_m / 8, rows, accumulate,
+  return cudaLaunchKernelEx(&lc, warp_rows ? row_checksum_kernel<1> : row_checksum_kernel<kChecksumWarps>, (const uint4*)y, (float*)sums, prob_m / 8, rows, accumulate,
                             row_map, first_row) == cudaSuccess
              ? TRB_OK
              : TRB_ERR_CUDA;
