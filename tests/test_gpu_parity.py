@@ -1076,40 +1076,79 @@ def test_lora_bgmv_with_base(cuda, K, N, rank, dtype):
     assert _lib().device_status(0) == 0
 
 
-@pytest.mark.parametrize("base_only", [False, True])
-def test_fused_calls_follow_what_produced_their_inputs(cuda, base_only):
-    """The one-call forms of ldmm and of sbmm with a base weight, whose kernels overlap each other, started right
-    behind kernels that produce x and the ids and let their successors start early: the same bits as with a
-    synchronisation before and after every call."""
+@pytest.mark.parametrize("call", ["ldmm", "sbmm", "lora_bgmv"])
+@pytest.mark.parametrize("T,K,N", [(96, 2048, 2048), (96, 2048, 11008), (1100, 2048, 2048)])
+def test_fused_calls_follow_what_produced_their_inputs(cuda, T, K, N, call):
+    """The one-call operators, whose kernels overlap each other, launched directly behind the kernel that produces x
+    and lets its successor start early (matmul_4bit_2_4; the ids lie ready, so nothing runs in between): the same bits
+    as with a synchronisation before and after every call.  Router and gather in one launch and in two, segments for
+    both grouped kernels, a base product that is split inside clusters and one with too many items for that."""
     ops = _ops()
-    K = N = 1024
-    T, D, M = 96, 12, 6
-    qs, metas, ss = packed(N, K, 128, seed=2, num=D)
+    D, M, n = 12, 6, 10
+    qs, metas, ss = ops.random_packed_deltas(D, K, N, groupsize=128, device=cuda, seed=2)
+    qp, mp, sp = ops.random_packed_deltas(1, K, K, groupsize=128, device=cuda, seed=3, scale_lo=0.0005, scale_hi=0.001)
     g = torch.Generator(cuda).manual_seed(4)
     w = (torch.randn(N, K, device=cuda, generator=g) * 0.02).half()
     A = (torch.randn(M, K, 16, device=cuda, generator=g) / 32).half()
     B = (torch.randn(M, 16, N, device=cuda, generator=g) / 4).half()
-    ids0 = torch.from_numpy(np.random.default_rng(0).integers(-1, D if base_only else M + D, T).astype(np.int32)).to(cuda)
-    x0 = torch.randn(T, K, device=cuda, generator=g).half()
+    count = {"lora_bgmv": M, "ldmm": M + D, "sbmm": D}[call]
+    p = 1.0 / np.arange(1, count + 2) ** 1.5             # a few long segments, several short ones, some rows without any
+    ids = [torch.from_numpy(np.random.default_rng(i).permutation(np.arange(-1, count))[
+        np.random.default_rng(i).choice(count + 1, T, p=p / p.sum())].astype(np.int32)).to(cuda) for i in range(n)]
+    xs = [torch.randn(T, K, device=cuda, generator=g).half() for _ in range(n)]
 
     def run(sync):
-        x, out = x0, []
-        for i in range(12):
+        out = []
+        for i in range(n):
             if sync:
                 torch.cuda.synchronize()
-            z = ops.matmul_4bit_2_4(qs[i % D], x, metas[i % D], ss[i % D])
-            ids = torch.roll(ids0, i)
+            z = ops.matmul_4bit_2_4(qp[0], xs[i], mp[0], sp[0])
             if sync:
                 torch.cuda.synchronize()
-            y = (ops.sbmm_4bit_2_4_native(qs, z, metas, ss, ids, base_weight=w) if base_only
-                 else ops.ldmm(ids, z, A, B, qs, metas, ss, base_weight=w))
-            x = (y / y.float().std()).half()
-            out.append(y)
+            if call == "ldmm":
+                out.append(ops.ldmm(ids[i], z, A, B, qs, metas, ss, base_weight=w))
+            elif call == "sbmm":
+                out.append(ops.sbmm_4bit_2_4_native(qs, z, metas, ss, ids[i], base_weight=w))
+            else:
+                out.append(ops.lora_bgmv(A, B, z, ids[i], base_weight=w))
         return out
 
-    a, b = run(True), run(False)
-    assert all(torch.equal(p, q) for p, q in zip(a, b))
+    expected = run(True)
+    for _ in range(3):
+        assert all(torch.equal(a, b) for a, b in zip(expected, run(False)))
     assert _lib().device_status(0) == 0
+
+
+def test_sbmm_in_two_phases(cuda):
+    """trb_sbmm_indexed_phase: router and gather (phase 1) and the grouped kernels (phase 2), on one stream and with
+    phase 1 on a stream of its own, against the one call."""
+    from triteia_b200._lib import lib, ptr
+    K, N, D, T = 256, 512, 5, 300
+    qs, metas, ss = packed(N, K, 128, seed=1, num=D)
+    g = torch.Generator(cuda).manual_seed(2)
+    x = torch.randn(T, K, dtype=torch.float16, device=cuda, generator=g)
+    y0 = torch.randn(T, N, dtype=torch.float16, device=cuda, generator=g)
+    idx = torch.from_numpy(np.random.default_rng(3).choice([-1, 0, 0, 0, 0, 1, 3, 4], T).astype(np.int32)).to(cuda)
+    nbytes = lib.trb_sbmm_indexed_scratch_bytes(T, K, D)
+    buf = torch.empty(nbytes, dtype=torch.uint8, device=cuda)
+
+    def call(y, phase, stream):
+        err = lib.trb_sbmm_indexed_phase(ptr(x), ptr(qs), ptr(metas), ptr(ss), ptr(idx), ptr(y), T, N, K, D, 0, 128, 1, ptr(buf),
+                                         nbytes, phase, 0, stream.cuda_stream)
+        assert err == 0
+
+    main, side = torch.cuda.current_stream(), torch.cuda.Stream()
+    whole, parts, two = y0.clone(), y0.clone(), y0.clone()
+    call(whole, 3, main)
+    call(parts, 1, main)
+    call(parts, 2, main)
+    side.wait_stream(main)
+    call(two, 1, side)
+    main.wait_stream(side)
+    call(two, 2, main)
+    assert torch.equal(whole, parts) and torch.equal(whole, two)
+    ref = sbmm_ref(qs, metas, ss, x, idx, None) + y0.float().cpu().numpy()
+    check(whole, ref)
 
 
 @pytest.mark.parametrize("T", [1, 31, 256, 257, 1024, 1025])
