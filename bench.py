@@ -311,7 +311,7 @@ def run_decode(args, world, rank, dev, barrier, dist):
     if world == 1:
         op = lambda xd, idd: ops.sbmm_4bit_2_4_native(qs, xd, metas, ss, idd)
         make_op = lambda: op
-        launches_per_step = 3   # router, row gather, grouped kernel
+        launches_per_step = 2   # router and row gather, grouped kernel
     else:
         exchange_kind, exchange = new_exchange()
         op = lambda xd, idd: exchange(xd, idd)
@@ -320,7 +320,10 @@ def run_decode(args, world, rank, dev, barrier, dist):
             """An exchange of its own (buffers, barriers) for a step that runs beside other steps."""
             _, ex = new_exchange()
             return lambda xd, idd: ex(xd, idd)
-        launches_per_step = 5 if exchange_kind == "p2p" else 6   # plan + pack, router + gather + grouped kernel (+ combine)
+        # pack (with the plan), router and gather (one launch up to 1024 rows of the receive buffer), the 8-token-tile
+        # kernel; the NCCL form also launches the 256-token-tile kernel and the combine
+        route = 1 if world * (TOKENS + 1) <= 1024 else 2
+        launches_per_step = 2 + route + (0 if exchange_kind == "p2p" else 2)
     step_resident = lambda: op(x_dev, idx_dev)
 
     for _ in range(max(3, args.warmup)):
@@ -793,9 +796,9 @@ def run_stack(args, world, rank, dev, barrier, dist, layers):
     return {"metric": "stack_tokens_per_s", "value": T_total / (t_step * 1e-3), "unit": UNIT, "n_gpus": world,
             "steps": steps, "ms_per_step": t_step, "timing": spread(times), "higher_is_better": True,
             "scaling": "strong", "dtype": "f16", "data": "synthetic",
-            # own kernels per pass: pack, router, one gather per input width, per linear the 256-token-tile launch,
-            # the 8-token-tile launch and the checksum, and the combine
-            "gpu_launches": steps * (5 + 3 * len(stack.LLAMA_7B_FUSED_LINEARS) * L),
+            # own kernels per pass: pack, router with the gather of the first input width, the gather of the second, per
+            # linear the 256-token-tile launch, the 8-token-tile launch and the checksum, and the combine
+            "gpu_launches": steps * (4 + 3 * len(stack.LLAMA_7B_FUSED_LINEARS) * L),
             "config": {"workload": f"stack-llama7b-linears-{L}layers-128deltas-512tok-zipf1.5-g128", "layers": L,
                        "tokens_total": T_total, "linears_per_pass": len(stack.LLAMA_7B_FUSED_LINEARS) * L, "linears": "qkv and gate_up fused as the reference's converter stores them", "ms_per_layer": t_step / L,
                        "distinct_deltas_touched": len(set(int(i) for i in ids_all)),
