@@ -468,8 +468,8 @@ extern "C" int trb_sbmm_indexed(const void* x, const void* qweights, const void*
 }
 
 // trb_sbmm_indexed in two calls, so that a caller can run the router and the row gather (phase 1:
-// they touch nothing but the scratch when accumulate != 0) on one stream beside other work -- the
-// base product of ldmm -- and the grouped kernels (phase 2) after both.  Same arguments and the
+// they touch nothing but the scratch when accumulate != 0) on one stream beside other work on
+// another, and the grouped kernels (phase 2) after both.  Same arguments and the
 // same scratch in both calls; phase 3 = trb_sbmm_indexed.
 extern "C" int trb_sbmm_indexed_phase(const void* x, const void* qweights, const void* metas, const void* scales,
                                       const void* indices, void* y, int num_tokens, int prob_m, int prob_k,

@@ -28,8 +28,9 @@
 // per stage.
 //
 // What bounds it (in-kernel cycle counters): a loop of latencies over the five stages, load about 1200 to 1500
-// cycles, decode 700, MMA and hand-back 500, that is 520 to 650 cycles per 128 K against 494 of the instruction at
-// 256 tokens; and for 256-token tiles the drain of the accumulator, about 4000 cycles an item.  The shared-memory
+// cycles, decode 700, MMA and hand-back 500: a fifth of that, 480 to 540 cycles, is the least a chunk of 128 K takes.
+// Measured 520 (narrow tiles) to 650 (256 tokens), where the instruction itself takes 494 at 256 tokens; and for
+// 256-token tiles the drain of the accumulator, about 4000 cycles an item.  The shared-memory
 // pipe would be next: 512 wavefronts of activations landing and read, 50 of packed weights, about 100 of decode;
 // weights in shared memory would add 256 and a proxy fence on the decode warps' chain.
 // Measured, whole calls (before: weights through shared memory, 64-K stages, every tile as 256 tokens, one
@@ -435,7 +436,7 @@ delta_gemm_tcsp_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_c
             }
             tc_st8(t_lane + Cfg::A_COL + 32 * st + 8 * s, v);
           }
-          tc_wait_st();
+          tc_wait_st();          // the stage's words have been used by now: no proxy fence before TMA may overwrite them
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive_cluster(aready_leader + st * 8);

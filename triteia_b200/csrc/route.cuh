@@ -268,9 +268,12 @@ route_kernel(const RouteSrc src, int T, int D, int W, int TT, int* __restrict__ 
 // sorted position of token t by itself (ids in smaller bins, and earlier ones in its own: T ids from L2, a compare
 // and a block sum) and copies its row, or zeroes its output row if it has no delta.  The two were a chain of two
 // kernels of 6 and 5 us at 100 tokens, each mostly launch and dependent loads.
-// Measured, whole calls: sbmm of 100 requests with a base weight 39.8 -> 33.1 us, ldmm of 100 requests 41.9 -> 39.0,
-// sbmm of 128 requests over 64 deltas 81.1 -> 80.4.
-// The T x T comparisons stay below a microsecond of L2 reads up to the limit.
+// Measured, whole calls: sbmm of 100 requests with a base weight 39.8 -> 33.1 us, ldmm of 100 requests 41.9 -> 39.0.
+// One call alone behind an L2 flush (two launches -> one): sbmm of 100 tokens over 64 deltas 77.7 -> 73.8, of 1024
+// tokens 197.1 -> 191.0; in a loop of decode calls there is no difference, because the router overlaps the call before.
+// The T x T comparisons stay below a microsecond of L2 reads up to the limit, also for ids that lie in an exchange
+// buffer, where each costs a division and a load: 4 ranks of 129 rows 82.3 -> 77.7, 2 of 512 rows 131.5 -> 127.1,
+// 16 of 64 rows over small deltas 41.0 -> 38.6.
 constexpr int kRouteGatherMax = 1024;
 constexpr int kRouteGatherSmem = 16 * 1024;     // of the router's shared memory, which every CTA of the launch gets
 
