@@ -15,6 +15,13 @@ def _inputs():
     return x, idx, q, meta, s
 
 
+@pytest.mark.parametrize("base", [(N - 128, K), (N + 128, K), (N, K - 64), (N, K + 64)])
+def test_sbmm_refuses_a_base_weight_that_does_not_fit_the_deltas(base):
+    x, idx, q, meta, s = _inputs()
+    with pytest.raises(RuntimeError, match="the deltas and inputs need"):
+        ops.sbmm_4bit_2_4_native(q, x, meta, s, idx, base_weight=torch.zeros(base, dtype=torch.float16))
+
+
 @pytest.mark.parametrize("base,a,b", [
     ((N - 128, K), (M, K, R), (M, R, N)),
     ((N, K - 64), (M, K, R), (M, R, N)),

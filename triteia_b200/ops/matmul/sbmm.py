@@ -119,7 +119,7 @@ def sbmm_4bit_2_4_native(qweights, xs, metas, ss, indices, base_weight=None):
     if not xs.is_contiguous():
         xs = xs.contiguous()
     if base_weight is not None:
-        if xs.dtype == torch.float16 and tuple(base_weight.shape) == (ss.shape[2], xs.shape[1]) and xs.shape[0] > 0:
+        if xs.dtype == torch.float16 and xs.shape[0] > 0:
             return base_indexed(xs, base_weight, qweights, metas, ss, indices)
         y = base_gemm(xs, base_weight)
         return sbmm_indexed(xs, qweights, metas, ss, indices, y=y)
