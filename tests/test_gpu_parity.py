@@ -850,9 +850,8 @@ def test_base_gemm_with_lora_expand(cuda, M, rank):
 @pytest.mark.parametrize("T,K,N,M", [(1, 1024, 264, 0), (100, 1088, 2048, 3), (70, 2048, 5120, 0), (256, 832, 11008, 2),
                                      (129, 1024, 512, 0), (2300, 128, 768, 0)])
 def test_base_gemm_split_and_order(cuda, T, K, N, M, dtype):
-    """Products with fewer items than CTA pairs, whose K range is shared inside a cluster (four pairs on an item,
-    two on one; uneven ranges; more pairs than token batches), with and
-    without LoRA chunks, writing and adding into y; and one with more token tiles than one group.  Against an fp32
+    """Products of one to many items, one of them shared by two CTA pairs along K, with and without LoRA chunks,
+    writing and adding into y; and one with more token tiles than one group.  Against an fp32
     torch statement: two roundings to the output type at most, so half of the tolerances of test_base_gemm."""
     from triteia_b200.ops.matmul._base import base_gemm
     g = torch.Generator(cuda).manual_seed(T + K + N)
@@ -871,11 +870,11 @@ def test_base_gemm_split_and_order(cuda, T, K, N, M, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
-@pytest.mark.parametrize("T,K,N,M", [(1, 1280, 264, 0), (1, 1344, 264, 0), (100, 1600, 2048, 3), (300, 1984, 4096, 0),
-                                     (300, 2112, 4096, 0)])
+@pytest.mark.parametrize("T,K,N,M", [(1, 1280, 264, 0), (1, 1344, 264, 0), (100, 1600, 2048, 3), (200, 1408, 520, 0),
+                                     (300, 1984, 4096, 0), (300, 2112, 4096, 0)])
 def test_base_gemm_on_both_sides_of_the_split_rule(cuda, T, K, N, M, dtype):
-    """20 chunks of K whole and 21 on four CTA pairs, 26 on four with LoRA chunks in the last range, 31 whole and 33 on two
-    pairs.  Element by element against 64 bits: one rounding to the type, a second one when added to y, fp32 sums."""
+    """20 chunks of K whole and 21 on four CTA pairs (more pairs than token batches), 26 on four with LoRA chunks in the
+    last range, 22 on four with seven token batches, 31 whole and 33 on two pairs.  Element by element against 64 bits: one rounding to the type, a second one when added to y, fp32 sums."""
     from triteia_b200.ops.matmul._base import base_gemm
     g = torch.Generator(cuda).manual_seed(T + K + N)
     x = torch.randn(T, K, device=cuda, generator=g).to(dtype)
