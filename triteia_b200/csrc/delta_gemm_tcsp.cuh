@@ -408,12 +408,12 @@ delta_gemm_tcsp_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_c
       for (int kc = 0; kc < k_chunks; ++kc) {
         if (turn == team) {
           mbar_wait(&full_bar[fb], phase, dead);
-          tc_fence_after();      // the stage's columns were read by MMAs: retired before TMA filled the stage again
           const uint32_t sb = smem_base + st * Cfg::STAGE_BYTES;
           uint32_t e[Cfg::SLABS];
 #pragma unroll
           for (int s = 0; s < Cfg::SLABS; ++s)
             e[s] = __byte_perm(lds32(sb + m_first + s * 512), lds32(sb + m_second + s * 512), msel);
+          tc_fence_after();      // the stage's columns were read by MMAs: retired before TMA filled the stage again
           tc_st4(t_lane + Cfg::META_COL + 4 * st, e[0], e[1], e[2], e[3]);
           uint32_t sc = 0;
           if (a.grouped) sc = lds16(sb + s_off) * 0x10001u;
